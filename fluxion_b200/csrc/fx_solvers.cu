@@ -16,6 +16,7 @@
 
 #include "fx_learned.cuh"
 #include "fx_points.cuh"
+#include "fx_reference.cuh"
 #include "fx_wcycle.cuh"
 
 using namespace fx;
@@ -550,87 +551,66 @@ int convert(fx_ctx *ctx, const S *src, D *dst, size_t n, const int *skip) {
     return launch_flat<0>(ctx, n, FlatConvert<S, D>{src, dst}, NoFin{}, skip, "mg_convert");
 }
 
-// Chebyshev smoother of the reference hierarchy (multigrid.rs:308-473): the first-kind
-// Chebyshev recurrence for D^-1 A with the bounds emax = 2, emin = 0.2 (D the level Laplacian's
-// diagonal) on three rotating vectors u, w0, w1, each step the reference's sequence of backend
-// ops (stencil apply, copy, axpy, scale, zero_boundaries) -- no inner products, no host sync.
-int chebyshev_smooth(fx_ctx *ctx, MgLevel &L, const fx_grid &g, const fx_stencil &s, const fx_boundaries &bc,
-                     size_t n) {
-    if (n == 0) return FX_OK;
-    const double emax = 2.0, emin = 0.1 * emax;
-    const double scale = 2.0 / (emax + emin);
-    const double alpha = 1.0 - scale * emin;
-    const double mu = 1.0 / alpha, omegaprod = 2.0 / alpha;
-    const double inv_dx2 = 1.0 / (L.dx * L.dx), inv_dy2 = 1.0 / (L.dy * L.dy);
-    const double inv_diag = -1.0 / (2.0 * inv_dx2 + 2.0 * inv_dy2);
-    double c_km1 = 1.0, c_k = mu;
-    FX_TRY(fx_apply_stencil(ctx, L.u, L.tmp, &g, &s, &bc));
-    FX_TRY(fx_copy(ctx, L.rhs, L.w0));
-    FX_TRY(fx_axpy(ctx, -1.0, L.tmp, L.w0));
-    FX_TRY(fx_scale(ctx, L.w0, scale * inv_diag));
-    FX_TRY(fx_axpy(ctx, 1.0, L.u, L.w0));
-    FX_TRY(fx_zero_boundaries(ctx, L.w0, L.rows, L.cols));
-    if (n == 1) return fx_copy(ctx, L.w0, L.u);
-    fx_buf *buf[3] = {L.u, L.w0, L.w1};
-    int km1 = 0, k = 1, kp1 = 2;
-    for (size_t i = 1; i < n; i++) {
-        FX_TRY(fx_apply_stencil(ctx, buf[k], L.tmp, &g, &s, &bc));
-        FX_TRY(fx_copy(ctx, L.rhs, buf[kp1]));
-        FX_TRY(fx_axpy(ctx, -1.0, L.tmp, buf[kp1]));
-        FX_TRY(fx_scale(ctx, buf[kp1], inv_diag));
-        const double c_kp1 = 2.0 * mu * c_k - c_km1;
-        const double omega = omegaprod * c_k / c_kp1;
-        FX_TRY(fx_scale(ctx, buf[kp1], omega * scale));
-        FX_TRY(fx_axpy(ctx, omega, buf[k], buf[kp1]));
-        FX_TRY(fx_axpy(ctx, 1.0 - omega, buf[km1], buf[kp1]));
-        FX_TRY(fx_zero_boundaries(ctx, buf[kp1], L.rows, L.cols));
-        c_km1 = c_k;
-        c_k = c_kp1;
-        const int t = km1;
-        km1 = k;
-        k = kp1;
-        kp1 = t;
-    }
-    if (k == 1) return fx_copy(ctx, L.w0, L.u);
-    if (k == 2) return fx_copy(ctx, L.w1, L.u);
-    return FX_OK;
-}
-
-// Reference-semantics cycle (multigrid.rs:188-230), built from the trait ops.
+// Reference-semantics cycle (multigrid.rs:188-230).  Each phase is the sequence of backend ops the
+// reference runs, fused where that leaves every value as it is (fx_reference.cu): consecutive
+// Jacobi sweeps in one launch, a Chebyshev step per launch (the first after a prolongation takes
+// the correction with it), residual and restriction in one.
 int reference_cycle(fx_mg *mg, fx_buf *x, const fx_buf *b, bool x_zero) {
     fx_ctx *ctx = mg->ctx;
     const int nl = (int)mg->lv.size();
     MgLevel &L0 = mg->lv[0];
-    FX_TRY(fx_copy(ctx, b, L0.rhs));
-    if (x_zero) FX_TRY(fx_fill(ctx, L0.u, 0.0));
-    else FX_TRY(fx_copy(ctx, x, L0.u));
-    auto smooth = [&](int l, size_t n) -> int {
+    FX_TRY(check_same(L0.rhs, b));
+    FX_TRY(check_same(L0.u, x));
+    // level 0 works on the caller's x and b where they are two buffers
+    const bool own = x->ptr == b->ptr;
+    if (own) {
+        FX_TRY(fx_copy(ctx, b, L0.rhs));
+        if (!x_zero) FX_TRY(fx_copy(ctx, x, L0.u));
+    }
+    auto u_of = [&](int l) { return (double *)(l == 0 && !own ? x->ptr : mg->lv[l].u->ptr); };
+    auto rhs_of = [&](int l) { return (const double *)(l == 0 && !own ? b->ptr : mg->lv[l].rhs->ptr); };
+    std::vector<StencilP> P(nl);
+    std::vector<BcP> B(nl);
+    for (int l = 0; l < nl; l++) {
+        const fx_stencil s{5, LAP_DR, LAP_DC, mg->lv[l].lap5};
+        FX_TRY(make_stencil(&s, &P[l]));
+        if (nl > 1 || mg->smoother == 1) FX_TRY(make_bc(&mg->bc, mg->lv[l].dx, mg->lv[l].dy, &B[l], true));
+    }
+    if (x_zero) FX_CUDA(cudaMemsetAsync(u_of(0), 0, L0.rows * L0.cols * sizeof(double), ctx->stream));
+    // smoothing on level l, after adding the prolongation of level l + 1's u when `correct`
+    auto smooth = [&](int l, size_t n, bool correct) -> int {
         MgLevel &L = mg->lv[l];
-        fx_grid g{L.rows, L.cols, L.dx, L.dy};
-        fx_stencil s{5, LAP_DR, LAP_DC, L.lap5};
-        if (mg->smoother == 1) return chebyshev_smooth(ctx, L, g, s, mg->bc, n);
-        for (size_t k = 0; k < n; k++) FX_TRY(fx_weighted_jacobi(ctx, L.u, L.rhs, mg->omega, &g, &s, &mg->bc));
-        return FX_OK;
+        if (correct) {
+            MgLevel &C = mg->lv[l + 1];
+            const fx_grid g{L.rows, L.cols, L.dx, L.dy}, cg{C.rows, C.cols, C.dx, C.dy};
+            if ((g.rows - 1) / 2 > cg.rows - 1 || (g.cols - 1) / 2 > cg.cols - 1)
+                return fail(FX_ERR_DIMENSION_MISMATCH, "prolong: fine grid maps outside the coarse grid");
+            if (mg->smoother == 0 || n == 0) {
+                fx_buf ub;
+                ub.ctx = ctx;
+                ub.ptr = u_of(l);
+                ub.len = L.rows * L.cols;
+                ub.owned = false;
+                FX_TRY(fx_prolong(ctx, C.u, &ub, &cg, &g));
+                correct = false;
+            }
+        }
+        if (mg->smoother == 1) {
+            const ChebLevel V{L.rows, L.cols, L.dx, L.dy, P[l], u_of(l), (double *)L.w0->ptr, (double *)L.w1->ptr, rhs_of(l)};
+            return cheb_smooth(ctx, V, correct ? (const double *)mg->lv[l + 1].u->ptr : nullptr,
+                               correct ? mg->lv[l + 1].cols : 0, n);
+        }
+        return lex5_sweeps<double>(ctx, u_of(l), rhs_of(l), L.rows, L.cols, L.lap5, mg->omega, 1.0 / L.lap5[0], n);
     };
     for (int l = 0; l < nl - 1; l++) {
         MgLevel &L = mg->lv[l], &C = mg->lv[l + 1];
-        FX_TRY(smooth(l, mg->n_pre));
-        fx_grid g{L.rows, L.cols, L.dx, L.dy}, cg{C.rows, C.cols, C.dx, C.dy};
-        fx_stencil s{5, LAP_DR, LAP_DC, L.lap5};
-        FX_TRY(fx_apply_stencil(ctx, L.u, L.tmp, &g, &s, &mg->bc));  // multigrid.rs:476-491
-        FX_TRY(fx_scale(ctx, L.tmp, -1.0));
-        FX_TRY(fx_axpy(ctx, 1.0, L.rhs, L.tmp));
-        FX_TRY(fx_restrict(ctx, L.tmp, C.rhs, &g, &cg));
-        FX_TRY(fx_fill(ctx, C.u, 0.0));
+        FX_TRY(smooth(l, mg->n_pre, false));
+        FX_TRY(ref_restrict_residual(ctx, u_of(l), rhs_of(l), L.rows, L.cols, P[l], B[l], (double *)C.rhs->ptr,
+                                     (double *)C.u->ptr, C.rows, C.cols));
     }
-    FX_TRY(smooth(nl - 1, mg->n_pre + mg->n_post + 10));
-    for (int l = nl - 2; l >= 0; l--) {
-        MgLevel &L = mg->lv[l], &C = mg->lv[l + 1];
-        fx_grid g{L.rows, L.cols, L.dx, L.dy}, cg{C.rows, C.cols, C.dx, C.dy};
-        FX_TRY(fx_prolong(ctx, C.u, L.u, &cg, &g));
-        FX_TRY(smooth(l, mg->n_post));
-    }
-    return fx_copy(ctx, L0.u, x);
+    FX_TRY(smooth(nl - 1, mg->n_pre + mg->n_post + 10, false));
+    for (int l = nl - 2; l >= 0; l--) FX_TRY(smooth(l, mg->n_post, true));
+    return own ? fx_copy(ctx, L0.u, x) : FX_OK;
 }
 
 }  // namespace

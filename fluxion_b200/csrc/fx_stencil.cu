@@ -3,6 +3,7 @@
 // smoothing primitives.  All grid kernels use the row-marching framework
 // (fx_internal.cuh): one HBM read per element of the marched field.
 #include "fx_points.cuh"
+#include "fx_reference.cuh"
 #include "fx_wcycle.cuh"
 
 using namespace fx;
@@ -447,6 +448,14 @@ int fx_weighted_jacobi(fx_ctx *ctx, fx_buf *x, const fx_buf *b, double omega, co
     }
     P.ne_ = s->n;
     const double inv_diag = 1.0 / diag;
+    // the five-point stencil in the Laplacian's entry order (what the reference's hierarchy smooths
+    // with) runs by diagonals; other stencils need the 2 r + c hyperplanes
+    if (lex5_order(s)) {
+        const double w[5] = {s->w[0], s->w[1], s->w[2], s->w[3], s->w[4]};
+        FX_DISPATCH(x->dtype, {
+            return lex5_sweeps<T>(ctx, (T *)x->ptr, (const T *)b->ptr, g->rows, g->cols, w, omega, inv_diag, 1);
+        });
+    }
     FX_DISPATCH(x->dtype, {
         k_lex_jacobi<T><<<1, 1024, 0, ctx->stream>>>((T *)x->ptr, (const T *)b->ptr, (int)g->rows,
                                                       (int)g->cols, P, omega, inv_diag);
