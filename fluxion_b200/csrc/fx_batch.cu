@@ -24,6 +24,7 @@
 #include <cmath>
 #include <vector>
 
+#include "fx_cdcycle.cuh"
 #include "fx_points.cuh"
 
 using namespace fx;
@@ -44,6 +45,12 @@ struct Chunk {
 struct Tile {
     int prob, ty, tx;
 };
+struct Strip {  // a warp's strip and row chunk of a fused level pass (fx_cdcycle.cuh)
+    int prob, strip, nstrips, r0, r1;
+};
+// Rows per strip item: a chunk marches 5 (down) or 3 (up) rows more than it owns, so long ones are
+// cheaper a row, and short ones balance better over the resident warps.
+constexpr int kStripRows = 64;
 
 // per (level, problem): offset into the level's arrays, side n (rows = cols = n), constants
 template <typename T>
@@ -614,39 +621,79 @@ __global__ void __launch_bounds__(256) k_bsweep2(const Tile *__restrict__ tiles,
     }
 }
 
-// The coarsest solve of one problem per block (k_cd_coarse's expressions): nsweeps sweeps from
-// zero in shared memory, the result written to u.
-template <typename T>
+// One warp per strip item of the level: the fused down and up passes of fx_cdcycle.cuh.  b is the
+// level's rhs (the FP64 vector r at level 0, whose layout the level-0 arrays share), z its result.
+template <typename T, typename TB, typename TZ>
+__device__ __forceinline__ CdLevelArgs<T, TB, TZ> strip_args(const LvlArgs<T> &a, const Lvl<T> *Lc, int p, T omega,
+                                                             const TB *b, T *x2, T *crhs, const T *e, TZ *z) {
+    const Lvl<T> &F = a.L[p], &C = Lc[p];
+    const long long o = F.off;
+    return CdLevelArgs<T, TB, TZ>{F.n, F.n, C.n, CdOp<T>{F.K, a.O.sigma, a.O.coeff, a.O.kap}, omega, b + o, a.vx + o,
+                                  a.vy + o, x2 + o, crhs ? crhs + C.off : nullptr, e ? e + C.off : nullptr,
+                                  z ? z + o : nullptr};
+}
+
+template <typename T, typename TB>
+__global__ void __launch_bounds__(kCdWarps * 32, cd_minb<T>()) k_bdown(const Strip *__restrict__ items, int n,
+                                                                       LvlArgs<T> a, const Lvl<T> *Lc, const TB *b,
+                                                                       T *x2, T *crhs, T omega) {
+    extern __shared__ __align__(16) unsigned char cd_smem[];
+    const int i = blockIdx.x * kCdWarps + (threadIdx.x >> 5);
+    if (i >= n) return;  // whole warps
+    const Strip it = items[i];
+    if (a.S[it.prob].halt || !FX_IN(it.r1 - 1, a.L[it.prob].n)) return;
+    cd_down_strip(strip_args<T, TB, TB>(a, Lc, it.prob, omega, b, x2, crhs, nullptr, nullptr), it.strip, it.r0, it.r1,
+                  cd_smem + (threadIdx.x >> 5) * cd_down_warp_smem<T, TB>());
+}
+
+template <typename T, typename TB, typename TZ>
+__global__ void __launch_bounds__(kCdWarps * 32, cd_minb<T>()) k_bup(const Strip *__restrict__ items, int n,
+                                                                     LvlArgs<T> a, const Lvl<T> *Lc, const TB *b,
+                                                                     T *x2, const T *e, TZ *z, int zero_ring, T omega) {
+    extern __shared__ __align__(16) unsigned char cd_smem[];
+    const int i = blockIdx.x * kCdWarps + (threadIdx.x >> 5);
+    if (i >= n) return;
+    const Strip it = items[i];
+    if (a.S[it.prob].halt || !FX_IN(it.r1 - 1, a.L[it.prob].n)) return;
+    cd_up_strip(strip_args<T, TB, TZ>(a, Lc, it.prob, omega, b, x2, nullptr, e, z), it.strip, it.nstrips, it.r0, it.r1,
+                zero_ring != 0, cd_smem + (threadIdx.x >> 5) * cd_up_warp_smem<T, TB>());
+}
+
+// The coarsest solve of one problem per block (k_cd_coarse's expressions and layout): nsweeps sweeps
+// from zero in shared memory, the result written to u.
+template <typename T, int PTS>
 __global__ void __launch_bounds__(1024) k_bcoarse(const int *__restrict__ probs, LvlArgs<T> a, T *ub, const T *bb,
                                                   T omega, int nsweeps) {
     const int prob = probs[blockIdx.x];
     if (a.S[prob].halt) return;
-    constexpr int kPts = 4;
     extern __shared__ unsigned char bsm[];
     const Lvl<T> &Lp = a.L[prob];
+    const ConvDiffC<T> K = Lp.K;
     const int rows = Lp.n, cols = Lp.n, n = rows * cols;
 #ifdef FX_CHECKED
     {
         unsigned dyn;
         asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn));
-        if (!(FX_IN(n - 1, kPts * (int)blockDim.x) && FX_IN(2LL * n - 1, dyn / sizeof(T)))) return;
+        if (!(FX_IN(n - 1, PTS * (int)blockDim.x) && FX_IN(2LL * n - 1, dyn / sizeof(T)))) return;
     }
 #endif
     T *s0 = reinterpret_cast<T *>(bsm);
     T *s1 = s0 + n;
     T *u = ub + Lp.off;
     const T *b = bb + Lp.off, *vx = a.vx + Lp.off, *vy = a.vy + Lp.off;
-    int idx[kPts];
-    bool inner[kPts];
-    T bv[kPts], dv[kPts];
+    int idx[PTS];
+    bool inner[PTS];
+    T bv[PTS], dv[PTS], xv[PTS], yv[PTS];
 #pragma unroll
-    for (int k = 0; k < kPts; k++) {
+    for (int k = 0; k < PTS; k++) {
         const int i = threadIdx.x + k * blockDim.x;
         idx[k] = i;
         const int r = i / cols, c = i % cols;
         inner[k] = i < n && r > 0 && c > 0 && r < rows - 1 && c < cols - 1;
         bv[k] = inner[k] ? b[i] : (T)0;
-        dv[k] = inner[k] ? (T)1 / bop_diag(a.O, Lp.K, vx[i], vy[i]) : (T)1;
+        xv[k] = inner[k] ? vx[i] : (T)0;
+        yv[k] = inner[k] ? vy[i] : (T)0;
+        dv[k] = inner[k] ? (T)1 / bop_diag(a.O, K, xv[k], yv[k]) : (T)1;
         if (i < n) {
             s0[i] = (T)0;
             s1[i] = (T)0;
@@ -657,7 +704,7 @@ __global__ void __launch_bounds__(1024) k_bcoarse(const int *__restrict__ probs,
         const T *src = (k & 1) ? s1 : s0;
         T *dst = (k & 1) ? s0 : s1;
 #pragma unroll
-        for (int q = 0; q < kPts; q++) {
+        for (int q = 0; q < PTS; q++) {
             if (!inner[q]) continue;
             const int i = idx[q];
             Nb<T> nb;
@@ -666,7 +713,7 @@ __global__ void __launch_bounds__(1024) k_bcoarse(const int *__restrict__ probs,
             nb.s = src[i + cols];
             nb.w = src[i - 1];
             nb.e = src[i + 1];
-            dst[i] = fx_fma(omega, (bv[q] - bop_apply(a.O, Lp.K, nb, vx[i], vy[i])) * dv[q], nb.c);
+            dst[i] = fx_fma(omega, (bv[q] - bop_apply(a.O, K, nb, xv[q], yv[q])) * dv[q], nb.c);
         }
         __syncthreads();
     }
@@ -733,6 +780,8 @@ struct fx_batch {
         int nsmooth = 0;
         Tile *tiles = nullptr;  // 32 x 32 tiles of the smoothing problems
         int ntiles = 0;
+        Strip *down = nullptr, *up = nullptr;  // strip items of the smoothing problems (fused passes)
+        int ndown = 0, nup = 0;
         int *coarse = nullptr;  // problems whose coarsest level this is
         int ncoarse = 0;
         int coarse_n = 0;       // their side (the largest)
@@ -857,6 +906,22 @@ int build_levels(fx_batch *B) {
         }
         FX_TRY(B->upload(&D.tiles, tiles));
         D.ntiles = (int)tiles.size();
+        if (B->n_pre == 2 && B->n_post == 2) {
+            std::vector<Strip> dn, up;
+            for (int p : smooth) {
+                const int n = side[l][p];
+                const int nd = (n - 1 + kCdOwnDown - 1) / kCdOwnDown, nu = (n - 1 + kCdOwnUp - 1) / kCdOwnUp;
+                for (int r0 = 0; r0 < n; r0 += kStripRows) {
+                    const int r1 = std::min(r0 + kStripRows, n);
+                    for (int s = 0; s < nd; s++) dn.push_back(Strip{p, s, nd, r0, r1});
+                    for (int s = 0; s < nu; s++) up.push_back(Strip{p, s, nu, r0, r1});
+                }
+            }
+            FX_TRY(B->upload(&D.down, dn));
+            FX_TRY(B->upload(&D.up, up));
+            D.ndown = (int)dn.size();
+            D.nup = (int)up.size();
+        }
         FX_TRY(B->upload(&D.coarse, coarse));
         D.ncoarse = (int)coarse.size();
         for (int p : coarse) D.coarse_n = std::max(D.coarse_n, side[l][p]);
@@ -926,15 +991,10 @@ int batch_cycle(fx_batch *B, double *z, const double *r) {
         cur[0] = (T *)z;
         oth[0] = (T *)B->kv[8];
         rhs[0] = (const T *)r;
-        FX_TRY((bflat<0>(B, B->d_chunk0, B->nchunk0, BfZero<T>{args(0), cur[0]}, NoFinB{}, "batch_zero")));
     } else {
         cur[0] = (T *)D0.u;
         oth[0] = (T *)D0.tmp;
         rhs[0] = (const T *)D0.rhs;
-        FX_TRY((bflat<0>(B, B->d_chunk0, B->nchunk0,
-                         BfCast<double, T>{B->d_lvl0_f64, (const Lvl<T> *)D0.lvl, r, (T *)D0.rhs, (T *)D0.u,
-                                           B->d_state},
-                         NoFinB{}, "batch_convert")));
     }
     for (int l = 1; l < nl; l++) {
         cur[l] = (T *)B->lv[l].u;
@@ -966,10 +1026,60 @@ int batch_cycle(fx_batch *B, double *z, const double *r) {
         const size_t n = (size_t)D.coarse_n * D.coarse_n;
         size_t t = ((n + 31) / 32) * 32;
         t = std::min<size_t>(std::max<size_t>(t, 32), 1024);
-        k_bcoarse<T><<<D.ncoarse, (unsigned)t, 2 * n * sizeof(T), ctx->stream>>>(D.coarse, args(l), cur[l], rhs[l],
-                                                                                  omega, (int)B->coarse_sweeps);
+        if (n <= 1024)
+            k_bcoarse<T, 1><<<D.ncoarse, (unsigned)t, 2 * n * sizeof(T), ctx->stream>>>(D.coarse, args(l), cur[l], rhs[l],
+                                                                                        omega, (int)B->coarse_sweeps);
+        else
+            k_bcoarse<T, 4><<<D.ncoarse, (unsigned)t, 2 * n * sizeof(T), ctx->stream>>>(D.coarse, args(l), cur[l], rhs[l],
+                                                                                        omega, (int)B->coarse_sweeps);
         return check_launch(ctx, "batch_coarse_solve");
     };
+    // two sweeps a leg: every level is the two strip passes, and level 0 reads r and writes z itself
+    // (an FP32 problem whose coarsest level is level 0 needs the cast vectors)
+    if (B->n_pre == 2 && B->n_post == 2 && !(B->dtype == FX_F32 && D0.ncoarse)) {
+        auto blocks = [](int n) { return (n + kCdWarps - 1) / kCdWarps; };
+        auto down = [&](int l, auto *b) -> int {
+            using TB = std::decay_t<decltype(*b)>;
+            const auto &D = B->lv[l], &C = B->lv[l + 1];
+            timing_pre(ctx, "batch_down");
+            k_bdown<T, TB><<<blocks(D.ndown), kCdWarps * 32, kCdWarps * cd_down_warp_smem<T, TB>(), ctx->stream>>>(
+                D.down, D.ndown, args(l), (const Lvl<T> *)C.lvl, b, oth[l], (T *)C.rhs, omega);
+            timing_post(ctx, 0.0);
+            return check_launch(ctx, "batch_down");
+        };
+        auto up = [&](int l, auto *b, auto *zl) -> int {
+            using TB = std::decay_t<decltype(*b)>;
+            using TZ = std::decay_t<decltype(*zl)>;
+            const auto &D = B->lv[l], &C = B->lv[l + 1];
+            constexpr size_t smem = kCdWarps * cd_up_warp_smem<T, TB>();
+            if (smem > 48 * 1024) FX_TRY(strip_smem_optin(k_bup<T, TB, TZ>, smem));
+            timing_pre(ctx, "batch_up");
+            k_bup<T, TB, TZ><<<blocks(D.nup), kCdWarps * 32, smem, ctx->stream>>>(
+                D.up, D.nup, args(l), (const Lvl<T> *)C.lvl, b, oth[l], cur[l + 1], zl, l == 0 ? 1 : 0, omega);
+            timing_post(ctx, 0.0);
+            return check_launch(ctx, "batch_up");
+        };
+        for (int l = 0; l < nl; l++) {
+            FX_TRY(coarse(l));  // problems whose coarsest level this is
+            if (l == nl - 1 || !B->lv[l].ndown) continue;
+            if (l == 0) FX_TRY(down(0, r));
+            else FX_TRY(down(l, rhs[l]));
+        }
+        for (int l = nl - 2; l >= 0; l--) {
+            if (!B->lv[l].nup) continue;
+            if (l == 0) FX_TRY(up(0, r, z));
+            else FX_TRY(up(l, rhs[l], cur[l]));
+        }
+        return FX_OK;
+    }
+    if (B->dtype == FX_F64) {
+        FX_TRY((bflat<0>(B, B->d_chunk0, B->nchunk0, BfZero<T>{args(0), cur[0]}, NoFinB{}, "batch_zero")));
+    } else {
+        FX_TRY((bflat<0>(B, B->d_chunk0, B->nchunk0,
+                         BfCast<double, T>{B->d_lvl0_f64, (const Lvl<T> *)D0.lvl, r, (T *)D0.rhs, (T *)D0.u,
+                                           B->d_state},
+                         NoFinB{}, "batch_convert")));
+    }
     for (int l = 0; l < nl; l++) {
         const auto &D = B->lv[l];
         FX_TRY(coarse(l));  // problems whose coarsest level this is

@@ -14,6 +14,7 @@
 #include <utility>
 #include <vector>
 
+#include "fx_cdcycle.cuh"
 #include "fx_learned.cuh"
 #include "fx_points.cuh"
 #include "fx_reference.cuh"
@@ -101,6 +102,8 @@ struct fx_precond {
     // true when apply(z, r, skip, true) writes every interior point of z from r alone and leaves
     // z's ring as it is, so a z whose ring is zero needs no zero-fill before each application
     virtual bool fills_from_zero(const fx_buf *) const { return false; }
+    // true when apply(z, r, skip, true) writes all of z, ring included, whatever it held
+    virtual bool writes_all() const { return false; }
 };
 
 namespace {
@@ -1054,7 +1057,7 @@ int cg_solve_impl(fx_cg *s, fx_buf *x, const fx_buf *b, double coeff, const Sten
     auto precondition = [&](bool first) -> int {
         const int st = pc->apply_pcg(&zb, &rb, halt, S, first);
         if (st != FX_ERR_UNSUPPORTED) return st;
-        FX_TRY(zero_fill<T>(ctx, z, n, halt));
+        if (!pc->writes_all()) FX_TRY(zero_fill<T>(ctx, z, n, halt));
         FX_TRY(pc->apply(&zb, &rb, halt, true));
         if (first) return launch_flat<1>(ctx, n, FlatDot<T>{r, z}, FinPcgRzInit{S}, halt, "pcg_rz");
         return launch_flat<1>(ctx, n, FlatDot<T>{r, z}, FinPcgRz{S}, halt, "pcg_rz");
@@ -1709,12 +1712,12 @@ int bicg_solve_impl(fx_bicgstab *s, fx_buf *x, const fx_buf *b, double coeff, co
     fx_buf sbuf{ctx, sv, n, FX_F64, false}, shb{ctx, sh, n, FX_F64, false};
     auto step = [&](size_t) -> int {
         FX_TRY(launch_flat<0>(ctx, n, FlatBicgP<T>{p, r, v, S}, NoFin{}, halt, "bicg_p"));
-        FX_TRY(zero_fill<T>(ctx, ph, n, halt));
+        if (!pc->writes_all()) FX_TRY(zero_fill<T>(ctx, ph, n, halt));
         FX_TRY(pc->apply(&phb, &pbuf, halt, true));
         FX_TRY((launch_pt<T, 1>(ctx, RR, CC, Ld1<T>{ph}, PtBicgV<T, MODE>{A, nullptr, v, rh}, FinBicgRv{S}, halt,
                                       "bicg_v")));
         FX_TRY(s_update(v));
-        FX_TRY(zero_fill<T>(ctx, sh, n, halt));
+        if (!pc->writes_all()) FX_TRY(zero_fill<T>(ctx, sh, n, halt));
         FX_TRY(pc->apply(&shb, &sbuf, halt, true));
         FX_TRY((launch_pt<T, 2>(ctx, RR, CC, Ld1<T>{sh}, PtBicgT<T, MODE>{A, tv, sv}, FinBicgT{S}, halt, "bicg_t")));
         return finish(ph, sh);
@@ -1872,7 +1875,7 @@ int gmres_solve_impl(fx_gmres *s, fx_buf *x, const fx_buf *b, double coeff, cons
         } else {
             FX_TRY((launch_pt<T, 0>(ctx, RR, CC, Ld1<T>{xp}, PtGmResid<T, MODE>{A, bp, w}, NoFin{}, nullptr, "gmres_resid")));
             fx_buf v0b{ctx, V[0], n, FX_F64, false};
-            FX_TRY(zero_fill<T>(ctx, V[0], n, nullptr));
+            if (!pc->writes_all()) FX_TRY(zero_fill<T>(ctx, V[0], n, nullptr));
             FX_TRY(pc->apply(&v0b, &wb, nullptr, true));
             T *v0 = V[0];
             FX_TRY(launch_flat<1>(ctx, n, FlatDot<T>{v0, v0}, FinSlot{dh}, nullptr, "gmres_beta"));
@@ -1910,7 +1913,7 @@ int gmres_solve_impl(fx_gmres *s, fx_buf *x, const fx_buf *b, double coeff, cons
                 FX_TRY((launch_pt<T, 0>(ctx, RR, CC, Ld1<T>{V[k]}, PtGmAv<T, MODE, false>{A, w, nullptr}, NoFin{}, nullptr,
                                               "gmres_av")));
                 fx_buf vk1{ctx, V[k + 1], n, FX_F64, false};
-                FX_TRY(zero_fill<T>(ctx, V[k + 1], n, nullptr));
+                if (!pc->writes_all()) FX_TRY(zero_fill<T>(ctx, V[k + 1], n, nullptr));
                 FX_TRY(pc->apply(&vk1, &wb, nullptr, true));
                 T *src = V[k + 1], *v0 = V[0];
                 FX_TRY(launch_flat<1>(ctx, n, FlatGmPcCopy<T>{w, src, v0}, FinSlot{dh + 0}, nullptr, "gmres_pc_copy"));
@@ -2381,7 +2384,7 @@ int fgmres_solve_impl(fx_fgmres *s, fx_buf *x, const fx_buf *b, double coeff, co
             }
             if (pc) {  // z_k = M^-1 v_k from a zero z_k
                 fx_buf zk{ctx, Z[k], n, FX_F64, false}, vk{ctx, V[k], n, FX_F64, false};
-                FX_TRY(zero_fill<T>(ctx, Z[k], n, nullptr));
+                if (!pc->writes_all()) FX_TRY(zero_fill<T>(ctx, Z[k], n, nullptr));
                 FX_TRY(pc->apply(&zk, &vk, nullptr, true));
             }
             double h_kp1_k = 0.0;
@@ -2911,13 +2914,17 @@ struct FlatCast {  // d = (D) s
 };
 
 // Coarsest level in one block: the iterate ping-pongs in shared memory, each thread keeps its
-// points' rhs and reciprocal diagonal in registers; every point value is FlatCdSweep's
-// expression.
-template <typename T>
+// points' rhs, coefficients and reciprocal diagonal in registers; every point value is
+// FlatCdSweep's expression.  The sweeps are a chain of dependent steps (a barrier, five shared
+// loads, ten dependent operations each), so a thread has one point (PTS = 1) wherever the grid fits
+// a block: a predicated-off point still issues its instructions.  On the 17 x 17 grid 200 FP64
+// sweeps took 51 us with four point slots per thread and the coefficients read in every sweep, and
+// 42 us now.
+template <typename T, int PTS>
 __global__ void __launch_bounds__(1024) k_cd_coarse(T *u, const T *__restrict__ b, int rows, int cols,
                                                     OpA<T, kModeCD> A, T omega, int nsweeps, const int *skip) {
+    grid_dep_enter();
     if (skip && *(volatile const int *)skip) return;
-    constexpr int kPts = 4;
     extern __shared__ unsigned char smem_raw[];
     T *s0 = reinterpret_cast<T *>(smem_raw);
     T *s1 = s0 + rows * cols;
@@ -2926,20 +2933,23 @@ __global__ void __launch_bounds__(1024) k_cd_coarse(T *u, const T *__restrict__ 
     {
         unsigned dyn;
         asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn));
-        if (!(FX_IN(n - 1, kPts * (int)blockDim.x) && FX_IN(2LL * n - 1, dyn / sizeof(T)))) return;
+        if (!(FX_IN(n - 1, PTS * (int)blockDim.x) && FX_IN(2LL * n - 1, dyn / sizeof(T)))) return;
     }
 #endif
-    int idx[kPts];
-    bool inner[kPts];
-    T bv[kPts], dv[kPts];
+    int idx[PTS];
+    bool inner[PTS];
+    T bv[PTS], dv[PTS], xv[PTS], yv[PTS], kv[PTS];
 #pragma unroll
-    for (int k = 0; k < kPts; k++) {
+    for (int k = 0; k < PTS; k++) {
         const int i = threadIdx.x + k * blockDim.x;
         idx[k] = i;
         const int r = i / cols, c = i % cols;
         inner[k] = i < n && r > 0 && c > 0 && r < rows - 1 && c < cols - 1;
         bv[k] = inner[k] ? b[i] : (T)0;
         dv[k] = inner[k] ? (T)1 / cd_diag(A, (size_t)i) : (T)1;  // 1 / diag
+        xv[k] = inner[k] ? A.vx[i] : (T)0;
+        yv[k] = inner[k] ? A.vy[i] : (T)0;
+        kv[k] = inner[k] && A.kappa ? A.kappa[i] : A.kap_s;
         if (i < n) {
             s0[i] = (T)0;
             s1[i] = (T)0;
@@ -2950,7 +2960,7 @@ __global__ void __launch_bounds__(1024) k_cd_coarse(T *u, const T *__restrict__ 
         const T *src = (k & 1) ? s1 : s0;
         T *dst = (k & 1) ? s0 : s1;
 #pragma unroll
-        for (int q = 0; q < kPts; q++) {
+        for (int q = 0; q < PTS; q++) {
             if (!inner[q]) continue;
             const int i = idx[q];
             Nb<T> nb;
@@ -2959,7 +2969,8 @@ __global__ void __launch_bounds__(1024) k_cd_coarse(T *u, const T *__restrict__ 
             nb.s = src[i + cols];
             nb.w = src[i - 1];
             nb.e = src[i + 1];
-            dst[i] = fx_fma(omega, (bv[q] - A.apply(false, nb, (size_t)i)) * dv[q], nb.c);
+            const T av = fx_fma(A.coeff, conv_diff_at<T>(A.K, nb, kv[q], xv[q], yv[q]), A.sigma * nb.c);
+            dst[i] = fx_fma(omega, (bv[q] - av) * dv[q], nb.c);
         }
         __syncthreads();
     }
@@ -2990,6 +3001,7 @@ struct fx_cdmg {
         fx_cdmg *mg = nullptr;
         int apply(fx_buf *z, const fx_buf *r, const int *skip, bool z_zero) override;
         int record(fx_buf *z, const fx_buf *r, const int *skip, bool z_zero);
+        bool writes_all() const override { return mg->fused(0, false) && !mg->lsm; }
     } view;
     // One application is a fixed sequence of launches for given (z, r, halt flag, stream).  With
     // replay on (fx_cdmg_set_replay), it is recorded into a CUDA graph the first time and
@@ -3035,6 +3047,23 @@ struct fx_cdmg {
             for (fx_buf *f : {L.u, L.rhs, L.tmp, L.vx, L.vy, L.kappa}) fx_free(f);
         fx_free(tmp0);
     }
+    // Levels of at most this many points keep the separate passes in a recorded cycle: replay is for
+    // hierarchies whose cycle is many launches, and what a recording holds there is what its users
+    // count.  The fused passes would save about 5 us of a replayed cycle (127 x 127: 78 against 71 us
+    // launched directly).
+    static constexpr size_t kReplaySeparate = 2048;
+    // whether level l smooths with the network in a learned cycle
+    bool learned_on(size_t l) const {
+        const size_t pts = lv[l].rows * lv[l].cols;
+        return l + 1 < lv.size() && pts >= lsm_min_points && (!lsm_max_points || pts <= lsm_max_points);
+    }
+    // whether level l runs as the fused passes of fx_cdcycle.cuh: they hold two sweeps a leg of a
+    // scalar-kappa operator (a kappa field would need a fourth ring row array; it keeps the
+    // separate passes, as other sweep counts do)
+    bool fused(size_t l, bool learned) const {
+        return n_pre == 2 && n_post == 2 && !op->kappa && l + 1 < lv.size() && !(learned && learned_on(l)) &&
+               !(replay && lv[l].rows * lv[l].cols <= kReplaySeparate);
+    }
     // The operator on level l: h doubled per level, the injected fields; level 0 of an F64
     // cycle reads the operator's own fields.
     template <typename T>
@@ -3056,26 +3085,48 @@ struct fx_cdmg {
 
 namespace {
 
+template <typename T, typename TB, typename TZ>
+CdLevelArgs<T, TB, TZ> cd_level_args(const fx_cdmg *mg, size_t l, const TB *b, T *x2, TZ *z) {
+    const CdLevel &L = mg->lv[l], &C = mg->lv[l + 1];
+    const auto A = mg->level_op<T>(l);
+    return CdLevelArgs<T, TB, TZ>{(int)L.rows, (int)L.cols, (int)C.cols, CdOp<T>{A.K, A.sigma, A.coeff, A.kap_s},
+                                  (T)mg->omega, b, A.vx, A.vy, x2, (T *)C.rhs->ptr, nullptr, z};
+}
+
+// z = one cycle of r from zero, computed in T.  Level 0 of an F32 cycle reads and writes the FP64
+// vectors directly when it is fused, and through the level's own F32 vectors otherwise.  z_zero: z
+// holds zeros (a fused level 0 writes all of z, a separate one starts from it).
 template <typename T>
-int cd_cycle(fx_cdmg *mg, T *x, const T *b, T *x_other, const int *skip, bool learned) {  // x holds zeros on entry
+int cd_cycle(fx_cdmg *mg, double *z, const double *r, const int *skip, bool learned, bool z_zero) {
     fx_ctx *ctx = mg->ctx;
     const int nl = (int)mg->lv.size();
+    constexpr bool F32 = sizeof(T) == 4;
+    const size_t n0 = mg->lv[0].rows * mg->lv[0].cols;
+    const bool fused0 = mg->fused(0, learned);
     std::vector<T *> cur(nl), oth(nl);
     std::vector<const T *> rhs(nl);
-    cur[0] = x;
-    oth[0] = x_other;
-    rhs[0] = b;
-    for (int l = 1; l < nl; l++) {
+    for (int l = F32 ? 0 : 1; l < nl; l++) {
         cur[l] = (T *)mg->lv[l].u->ptr;
         oth[l] = (T *)mg->lv[l].tmp->ptr;
         rhs[l] = (const T *)mg->lv[l].rhs->ptr;
+    }
+    if constexpr (F32) {
+        if (!fused0) {
+            FX_TRY((launch_flat<0>(ctx, n0, FlatCast<double, float>{r, (float *)mg->lv[0].rhs->ptr}, NoFin{}, skip,
+                                   "cdmg_convert")));
+            FX_TRY(zero_fill<float>(ctx, cur[0], n0, skip));
+        }
+    } else {
+        cur[0] = z;
+        oth[0] = (T *)mg->tmp0->ptr;
+        rhs[0] = r;
+        if (!fused0 && !z_zero) FX_TRY(zero_fill<double>(ctx, z, n0, skip));
     }
     const T omega = (T)mg->omega;
     auto smooth = [&](int l, size_t n) -> int {
         const CdLevel &L = mg->lv[l];
         const auto A = mg->level_op<T>(l);
-        if (learned && l < nl - 1 && L.rows * L.cols >= mg->lsm_min_points &&
-            (!mg->lsm_max_points || L.rows * L.cols <= mg->lsm_max_points)) {  // in place; oth[l] holds q
+        if (learned && mg->learned_on(l)) {  // in place; oth[l] holds q
             for (size_t k = 0; k < n; k++)
                 FX_TRY(lsm_step<T>(ctx, mg->lsm, A, cur[l], oth[l], rhs[l], omega, L.rows, L.cols, L.dx, L.dy,
                                    mg->d_lsm_scale, skip));
@@ -3101,34 +3152,61 @@ int cd_cycle(fx_cdmg *mg, T *x, const T *b, T *x_other, const int *skip, bool le
     };
     for (int l = 0; l < nl - 1; l++) {
         const CdLevel &L = mg->lv[l], &Cl = mg->lv[l + 1];
-        FX_TRY(smooth(l, mg->n_pre));
-        FX_TRY((launch_flat<0>(ctx, L.rows * L.cols,
-                               FlatCdResid<T>{mg->level_op<T>(l), cur[l], oth[l], rhs[l], L.rows, L.cols}, NoFin{},
-                               skip, "cdmg_residual")));
-        FX_TRY(restrict_fw<T>(ctx, oth[l], (T *)Cl.rhs->ptr, L.cols, Cl.rows, Cl.cols, skip));
-        FX_TRY(zero_fill<T>(ctx, cur[l + 1], Cl.rows * Cl.cols, skip));
+        if (mg->fused(l, learned)) {  // x2 goes to oth[l]
+            if (F32 && l == 0)
+                FX_TRY((launch_cd_down<T, double, double>(ctx, cd_level_args<T, double, double>(mg, 0, r, oth[0], z), skip)));
+            else
+                FX_TRY((launch_cd_down<T, T, T>(ctx, cd_level_args<T, T, T>(mg, l, rhs[l], oth[l], cur[l]), skip)));
+        } else {
+            FX_TRY(smooth(l, mg->n_pre));
+            FX_TRY((launch_flat<0>(ctx, L.rows * L.cols,
+                                   FlatCdResid<T>{mg->level_op<T>(l), cur[l], oth[l], rhs[l], L.rows, L.cols}, NoFin{},
+                                   skip, "cdmg_residual")));
+            FX_TRY(restrict_fw<T>(ctx, oth[l], (T *)Cl.rhs->ptr, L.cols, Cl.rows, Cl.cols, skip));
+        }
+        const bool coarsest = l + 1 == nl - 1;
+        const size_t nc = Cl.rows * Cl.cols;
+        // the next level's iterate starts from zero: a fused level and the one-block solve do so themselves
+        if (coarsest ? !(coarse_fits(nc, sizeof(T)) && mg->coarse_sweeps > 0) : !mg->fused(l + 1, learned))
+            FX_TRY(zero_fill<T>(ctx, cur[l + 1], nc, skip));
     }
     {
         const int l = nl - 1;
         const CdLevel &L = mg->lv[l];
         const size_t n = L.rows * L.cols;
         if (coarse_fits(n, sizeof(T)) && mg->coarse_sweeps > 0) {
-            k_cd_coarse<T><<<1, coarse_threads(n), 2 * n * sizeof(T), ctx->stream>>>(
-                cur[l], rhs[l], (int)L.rows, (int)L.cols, mg->level_op<T>(l), omega, (int)mg->coarse_sweeps, skip);
-            FX_TRY(check_launch(ctx, "cdmg_coarse_solve"));
+            auto solve = [&](auto kernel) {
+                launch_pdl(ctx, kernel, dim3(1), dim3((unsigned)coarse_threads(n)), 2 * n * sizeof(T), cur[l], rhs[l],
+                           (int)L.rows, (int)L.cols, mg->level_op<T>(l), omega, (int)mg->coarse_sweeps, skip);
+                return check_launch(ctx, "cdmg_coarse_solve");
+            };
+            if (n <= 1024) FX_TRY(solve(k_cd_coarse<T, 1>));
+            else FX_TRY(solve(k_cd_coarse<T, 4>));
         } else {
             FX_TRY(smooth(l, mg->coarse_sweeps));
         }
     }
     for (int l = nl - 2; l >= 0; l--) {
         const CdLevel &L = mg->lv[l], &Cl = mg->lv[l + 1];
+        if (mg->fused(l, learned)) {
+            if (F32 && l == 0) {
+                auto a = cd_level_args<T, double, double>(mg, 0, r, oth[0], z);
+                a.e = cur[1];
+                FX_TRY((launch_cd_up<T, double, double>(ctx, a, true, skip)));
+            } else {
+                auto a = cd_level_args<T, T, T>(mg, l, rhs[l], oth[l], cur[l]);
+                a.e = cur[l + 1];
+                FX_TRY((launch_cd_up<T, T, T>(ctx, a, l == 0, skip)));
+            }
+            continue;
+        }
         FX_TRY(prolong_bilinear<T>(ctx, cur[l + 1], cur[l], Cl.cols, L.rows, L.cols, skip));
         FX_TRY(smooth(l, mg->n_post));
     }
-    if (cur[0] != x) {
-        const CdLevel &L0 = mg->lv[0];
-        FX_CUDA(cudaMemcpyAsync(x, cur[0], L0.rows * L0.cols * sizeof(T), cudaMemcpyDeviceToDevice, ctx->stream));
-    }
+    if (F32 && !fused0)
+        return launch_flat<0>(ctx, n0, FlatCast<T, double>{cur[0], z}, NoFin{}, skip, "cdmg_convert");
+    if (!F32 && (const void *)cur[0] != (const void *)z)
+        FX_CUDA(cudaMemcpyAsync(z, cur[0], n0 * sizeof(T), cudaMemcpyDeviceToDevice, ctx->stream));
     return FX_OK;
 }
 
@@ -3185,16 +3263,9 @@ int fx_cdmg::View::record(fx_buf *z, const fx_buf *r, const int *skip, bool z_ze
         return fail(FX_ERR_DIMENSION_MISMATCH, "conv-diff multigrid: vectors must be F64 fields of the operator's grid");
     if (z->ptr == r->ptr) return fail(FX_ERR_INVALID_ARGUMENT, "z and r must be distinct");
     auto run = [&](bool learned, const int *sk, bool zz) -> int {
-        if (mg->dtype == FX_F32) {  // r -> F32, the cycle in F32, z = its F64 image
-            float *x = (float *)L0.u->ptr, *b = (float *)L0.rhs->ptr;
-            FX_TRY((launch_flat<0>(ctx, n, FlatCast<double, float>{(const double *)r->ptr, b}, NoFin{}, sk,
-                                   "cdmg_convert")));
-            FX_TRY(zero_fill<float>(ctx, x, n, sk));
-            FX_TRY(cd_cycle<float>(mg, x, b, (float *)L0.tmp->ptr, sk, learned));
-            return launch_flat<0>(ctx, n, FlatCast<float, double>{x, (double *)z->ptr}, NoFin{}, sk, "cdmg_convert");
-        }
-        if (!zz) FX_TRY(zero_fill<double>(ctx, (double *)z->ptr, z->len, sk));
-        return cd_cycle<double>(mg, (double *)z->ptr, (const double *)r->ptr, (double *)mg->tmp0->ptr, sk, learned);
+        double *zp = (double *)z->ptr;
+        const double *rp = (const double *)r->ptr;
+        return mg->dtype == FX_F32 ? cd_cycle<float>(mg, zp, rp, sk, learned, zz) : cd_cycle<double>(mg, zp, rp, sk, learned, zz);
     };
     if (!mg->lsm) return run(false, skip, z_zero);
     // the learned cycle, its check, and the plain cycle where the check failed (all on the device)
