@@ -1736,7 +1736,11 @@ struct fx_gmres : SolverBase {
     double *h_h_dev = nullptr;  // its device address
     std::vector<double> hh, cc, ss, grs;
     std::vector<fx_buf *> vv;  // m+1 basis vectors (bufs[0..m]); w = bufs[m+1]
+    double *d_mgs = nullptr;      // two-pass Gram-Schmidt: the basis' Gram rows, then block partials
+    unsigned *d_mgs_ticket = nullptr;
     ~fx_gmres() {
+        if (d_mgs) cudaFree(d_mgs);
+        if (d_mgs_ticket) cudaFree(d_mgs_ticket);
         if (d_h) cudaFree(d_h);
         if (h_h) cudaFreeHost(h_h);
     }
@@ -1816,6 +1820,244 @@ struct FlatGmMgs {  // w -= h_j v_j; reduction w.v_{j+1} (or w.w after the last)
         else csum_add_prod(acc[0], (double)wv, (double)wv);
     }
 };
+
+// ------------------------------------------------ modified Gram-Schmidt in two passes
+//
+// Modified Gram-Schmidt subtracts h_j v_j from w one vector at a time, h_j = v_j . w of the updated
+// w: a pass over w per basis vector, 32 B/point each (105 us at 4097 x 4097, at the HBM rate; 48 % of a
+// convection-diffusion FGMRES(30) solve).  In exact arithmetic h is the solution of (I + L) h = V^T w
+// with L the strictly lower triangle of V^T V (the low-synchronisation form of the method;
+// Swirydowicz, Langou, Ananthan, Yang, Thomas 2021), so two passes over the basis give the same
+// coefficients up to rounding, 16 B/point per vector:
+//   dots:   s_j = v_j . w and row k of L, v_j . v_k, in one pass; the last block solves for h;
+//   update: w -= sum_j h_j v_j, element by element in MGS's order, and ||w||^2.
+// s_j and ||w||^2 are sums of exact products, as MGS's dots; the entries of L (of rounding size, and
+// multiplying h) are per-thread fma partials folded compensated.
+//
+// Dots: a block takes a group of up to 8 basis vectors (its threads hold 8 compensated sums) over a
+// share of the elements, so w and v_k are read once per group, mostly from L2; groups are of equal
+// size, and their registers are capped for two blocks per SM (three for up to 5 vectors): 1.44 ms an
+// iteration of FGMRES(30) with the fused cycle at 4097 x 4097 without the cap, 1.35 with it.  Against
+// a pass per vector: 1.84 ms an iteration there, 42 against 92 us for GMRES(30) at 129 x 131 (two
+// launches a step instead of k + 1), 249 against 446 at 2049 x 2049.  Two sums per 8 bytes read are
+// half of the FP64 rate at the HBM rate; both passes run within 10 % of it.
+constexpr int kMgsMax = 32;   // basis vectors (above, and for one vector, a pass per vector)
+constexpr int kMgsGroup = 8;  // vectors per block
+
+struct MgsArgs {
+    double *w;
+    const double *v[kMgsMax];
+    int kb;       // basis vectors v_0 .. v_{kb-1}
+    int ng;       // vector groups
+    double *L;    // [kMgsMax][kMgsMax]: rows of V^T V
+    double *part; // [blocks][4 kMgsGroup]: per vector (s, c) of w . v_j, then (s, c) of v_j . v_k
+    unsigned *ticket;
+    double *h;    // [kb + 1]: the coefficients, then ||w||^2
+};
+
+template <int GS>
+__global__ void __launch_bounds__(kBlock, GS >= 6 ? 2 : 3) k_mgs_dots(size_t n, MgsArgs a) {
+    grid_dep_enter();
+    const int grp = blockIdx.x % a.ng, lb = blockIdx.x / a.ng;
+    const int nbg = (gridDim.x - grp + a.ng - 1) / a.ng;  // blocks of this group
+    const int j0 = (int)((long long)a.kb * grp / a.ng), j1 = (int)((long long)a.kb * (grp + 1) / a.ng);
+    const double *v[GS];
+#pragma unroll
+    for (int q = 0; q < GS; q++) v[q] = a.v[min(j0 + q, j1 - 1)];
+    const double *vk = a.v[a.kb - 1];
+    CSum acc[2 * GS];
+#pragma unroll
+    for (int q = 0; q < 2 * GS; q++) acc[q] = CSum{0.0, 0.0};
+    const size_t stride = (size_t)nbg * kBlock;
+    size_t i = (size_t)lb * kBlock + threadIdx.x;
+    for (; i + stride < n; i += 2 * stride) {  // two elements' loads in flight
+        double x[2], y[2], e[2][GS];
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            x[u] = a.w[i + u * stride];
+            y[u] = vk[i + u * stride];
+#pragma unroll
+            for (int q = 0; q < GS; q++) e[u][q] = v[q][i + u * stride];
+        }
+#pragma unroll
+        for (int u = 0; u < 2; u++)
+#pragma unroll
+            for (int q = 0; q < GS; q++) {
+                csum_add_prod(acc[q], e[u][q], x[u]);
+                csum_fma(acc[GS + q], e[u][q], y[u]);
+            }
+    }
+    if (i < n) {
+        const double x = a.w[i], y = vk[i];
+#pragma unroll
+        for (int q = 0; q < GS; q++) {
+            const double e = v[q][i];
+            csum_add_prod(acc[q], e, x);
+            csum_fma(acc[GS + q], e, y);
+        }
+    }
+    block_reduce<2 * GS>(acc);
+    __shared__ bool is_last;
+    if (threadIdx.x == 0) {
+        double *p = a.part + (size_t)blockIdx.x * (4 * kMgsGroup);
+#pragma unroll
+        for (int q = 0; q < GS; q++) {
+            p[4 * q] = acc[q].s;
+            p[4 * q + 1] = acc[q].c;
+            p[4 * q + 2] = acc[GS + q].s;
+            p[4 * q + 3] = acc[GS + q].c;
+        }
+        __threadfence();
+        is_last = atomicAdd(a.ticket, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!is_last) return;
+    __threadfence();
+    // the last block: fold each vector's partials in block order (a warp per vector), then solve
+    __shared__ double s[kMgsMax], Lm[kMgsMax][kMgsMax + 1];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, kb = a.kb;
+    for (int t = threadIdx.x; t < (kb - 1) * kMgsMax; t += kBlock) Lm[t / kMgsMax][t % kMgsMax] = a.L[t];
+    for (int j = wid; j < kb; j += kBlock / 32) {
+        int g = 0;
+        while ((int)((long long)kb * (g + 1) / a.ng) <= j) g++;
+        const int q = j - (int)((long long)kb * g / a.ng), nb = ((int)gridDim.x - g + a.ng - 1) / a.ng;
+        CSum d{0.0, 0.0}, l{0.0, 0.0};
+        for (int b = lane; b < nb; b += 32) {
+            const double *p = a.part + (size_t)(g + b * a.ng) * (4 * kMgsGroup) + 4 * q;
+            d = csum_merge(d, CSum{__ldcg(p), __ldcg(p + 1)});
+            l = csum_merge(l, CSum{__ldcg(p + 2), __ldcg(p + 3)});
+        }
+        for (int off = 16; off > 0; off >>= 1) {
+            CSum o;
+            o.s = __shfl_down_sync(0xffffffffu, d.s, off);
+            o.c = __shfl_down_sync(0xffffffffu, d.c, off);
+            d = csum_merge(d, o);
+            o.s = __shfl_down_sync(0xffffffffu, l.s, off);
+            o.c = __shfl_down_sync(0xffffffffu, l.c, off);
+            l = csum_merge(l, o);
+        }
+        if (lane == 0) {
+            s[j] = csum_value(d);
+            if (j < kb - 1) {
+                const double lv = csum_value(l);
+                Lm[kb - 1][j] = lv;
+                a.L[(kb - 1) * kMgsMax + j] = lv;
+            }
+        }
+    }
+    __syncthreads();
+    if (wid == 0) {  // h_j = s_j - sum_{i < j} L_ji h_i, a column at a time
+        double r = lane < kb ? s[lane] : 0.0;
+        for (int i = 0; i + 1 < kb; i++) {
+            const double hi = __shfl_sync(0xffffffffu, r, i);
+            if (lane > i && lane < kb) r = fma(-Lm[lane][i], hi, r);
+        }
+        if (lane < kb) a.h[lane] = r;
+    }
+    if (threadIdx.x == 0) *a.ticket = 0u;
+}
+
+// w -= sum_j h_j v_j, ||w||^2 -> h[kb]
+__global__ void __launch_bounds__(kBlock) k_mgs_update(size_t n, MgsArgs a, RedArgs<1> ra) {
+    grid_dep_enter();
+    __shared__ double c[kMgsMax];
+    __shared__ const double *vp[kMgsMax];
+    if (threadIdx.x < kMgsMax) {
+        c[threadIdx.x] = threadIdx.x < a.kb ? -a.h[threadIdx.x] : 0.0;
+        vp[threadIdx.x] = a.v[min((int)threadIdx.x, a.kb - 1)];
+    }
+    __syncthreads();
+    constexpr int kU = 2, kB = 8;
+    CSum acc[1] = {CSum{0.0, 0.0}};
+    const size_t stride = (size_t)gridDim.x * kBlock;
+    for (size_t i0 = (size_t)blockIdx.x * kBlock + threadIdx.x; i0 < n; i0 += kU * stride) {
+        double wv[kU];
+        bool in[kU];
+#pragma unroll
+        for (int u = 0; u < kU; u++) {
+            in[u] = i0 + u * stride < n;
+            wv[u] = in[u] ? a.w[i0 + u * stride] : 0.0;
+        }
+        for (int j0 = 0; j0 < a.kb; j0 += kB) {
+            double e[kU][kB];
+#pragma unroll
+            for (int t = 0; t < kB; t++) {
+                const bool on = j0 + t < a.kb;  // uniform
+#pragma unroll
+                for (int u = 0; u < kU; u++) e[u][t] = on && in[u] ? vp[j0 + t][i0 + u * stride] : 0.0;
+            }
+#pragma unroll
+            for (int t = 0; t < kB; t++)
+                if (j0 + t < a.kb) {
+                    const double ct = c[j0 + t];
+#pragma unroll
+                    for (int u = 0; u < kU; u++) wv[u] = fma(ct, e[u][t], wv[u]);
+                }
+        }
+#pragma unroll
+        for (int u = 0; u < kU; u++)
+            if (in[u]) {
+                a.w[i0 + u * stride] = wv[u];
+                csum_add_prod(acc[0], wv[u], wv[u]);
+            }
+    }
+    grid_reduce<1>(acc, ra, FinSlot{a.h + a.kb});
+}
+
+template <int GS>
+int launch_mgs_dots(fx_ctx *ctx, size_t n, MgsArgs &a) {
+    static std::atomic<int> occ{0};
+    const size_t cap = (size_t)band_capacity(ctx, k_mgs_dots<GS>, occ, kBlock);
+    size_t blocks = (size_t)a.ng * ((n + 2 * kBlock - 1) / (2 * kBlock));
+    if (blocks > cap) blocks = cap;
+    if (blocks > (size_t)ctx->num_sms * 8) blocks = (size_t)ctx->num_sms * 8;  // rows of `part`
+    if (blocks < (size_t)a.ng) blocks = (size_t)a.ng;
+    timing_pre(ctx, "gmres_mgs_dots");
+    launch_pdl(ctx, k_mgs_dots<GS>, (int)blocks, kBlock, 0, n, a);
+    timing_post(ctx, (double)n, (double)n * 8.0 * (a.kb + 1));
+    return check_launch(ctx, "gmres_mgs_dots");
+}
+
+// Orthogonalise w against V[0 .. kb), kb >= 2: dh[0 .. kb) the coefficients, dh[kb] = ||w||^2.
+int mgs_two_pass(fx_gmres *s, size_t n, double *w, const std::vector<double *> &V, size_t kb, double *dh) {
+    fx_ctx *ctx = s->ctx;
+    MgsArgs a{};
+    a.w = w;
+    for (size_t j = 0; j < kb; j++) a.v[j] = V[j];
+    a.kb = (int)kb;
+    a.ng = (int)((kb + kMgsGroup - 1) / kMgsGroup);
+    a.L = s->d_mgs;
+    a.part = s->d_mgs + kMgsMax * kMgsMax;
+    a.ticket = s->d_mgs_ticket;
+    a.h = dh;
+    switch ((kb + a.ng - 1) / a.ng) {  // the largest group's size
+        case 2: FX_TRY(launch_mgs_dots<2>(ctx, n, a)); break;
+        case 3: FX_TRY(launch_mgs_dots<3>(ctx, n, a)); break;
+        case 4: FX_TRY(launch_mgs_dots<4>(ctx, n, a)); break;
+        case 5: FX_TRY(launch_mgs_dots<5>(ctx, n, a)); break;
+        case 6: FX_TRY(launch_mgs_dots<6>(ctx, n, a)); break;
+        case 7: FX_TRY(launch_mgs_dots<7>(ctx, n, a)); break;
+        default: FX_TRY(launch_mgs_dots<8>(ctx, n, a)); break;
+    }
+    static std::atomic<int> occ{0};
+    const size_t cap = (size_t)band_capacity(ctx, k_mgs_update, occ, kBlock);
+    size_t blocks = std::min(cap, (n + 2 * kBlock - 1) / (2 * kBlock));
+    if (blocks > (size_t)kMaxRedBlocks) blocks = kMaxRedBlocks;
+    timing_pre(ctx, "gmres_mgs_update");
+    launch_pdl(ctx, k_mgs_update, (int)blocks, kBlock, 0, n, a, red_args<1>(ctx));
+    timing_post(ctx, (double)n, (double)n * 8.0 * (kb + 2));
+    return check_launch(ctx, "gmres_mgs_update");
+}
+
+// scratch of the two-pass form, made with the solver
+int mgs_alloc(fx_gmres *s) {
+    const size_t words = (size_t)kMgsMax * kMgsMax + (size_t)s->ctx->num_sms * 8 * 4 * kMgsGroup;
+    FX_CUDA(cudaMalloc(&s->d_mgs, words * sizeof(double)));
+    FX_CUDA(cudaMemset(s->d_mgs, 0, words * sizeof(double)));
+    FX_CUDA(cudaMalloc(&s->d_mgs_ticket, sizeof(unsigned)));
+    FX_CUDA(cudaMemset(s->d_mgs_ticket, 0, sizeof(unsigned)));
+    return FX_OK;
+}
 
 template <int MODE>
 int gmres_solve_impl(fx_gmres *s, fx_buf *x, const fx_buf *b, double coeff, const StencilP &P, fx_precond *pc) {
@@ -1904,9 +2146,13 @@ int gmres_solve_impl(fx_gmres *s, fx_buf *x, const fx_buf *b, double coeff, cons
                 finished = true;
                 break;
             }
-            // w = A v_k (+ left preconditioning), then modified Gram-Schmidt with every dot
-            // fused into the preceding AXPY
-            if (!pc) {
+            // w = A v_k (+ left preconditioning), then modified Gram-Schmidt: in two passes over the
+            // basis, or with every dot fused into the preceding AXPY
+            const bool two = k >= 1 && k < (size_t)kMgsMax;
+            if (!pc && two) {
+                FX_TRY((launch_pt<T, 0>(ctx, RR, CC, Ld1<T>{V[k]}, PtGmAv<T, MODE, false>{A, w, nullptr}, NoFin{}, nullptr,
+                                              "gmres_av")));
+            } else if (!pc) {
                 FX_TRY((launch_pt<T, 1>(ctx, RR, CC, Ld1<T>{V[k]}, PtGmAv<T, MODE, true>{A, w, V[0]}, FinSlot{dh + 0}, nullptr,
                                               "gmres_av")));
             } else {
@@ -1918,7 +2164,8 @@ int gmres_solve_impl(fx_gmres *s, fx_buf *x, const fx_buf *b, double coeff, cons
                 T *src = V[k + 1], *v0 = V[0];
                 FX_TRY(launch_flat<1>(ctx, n, FlatGmPcCopy<T>{w, src, v0}, FinSlot{dh + 0}, nullptr, "gmres_pc_copy"));
             }
-            for (size_t j = 0; j <= k; j++) {
+            if (two) FX_TRY(mgs_two_pass(s, n, w, V, k + 1, dh));
+            for (size_t j = 0; !two && j <= k; j++) {
                 const T *vj = V[j];
                 const T *vn = j < k ? V[j + 1] : nullptr;
                 const double *hj = dh + j;
@@ -2410,6 +2657,13 @@ int fgmres_solve_impl(fx_fgmres *s, fx_buf *x, const fx_buf *b, double coeff, co
                 const double *hv = s->h_h;
                 for (size_t j = 0; j <= k; j++) H(j, k) = hv[j] + hv[m + 2 + j];
                 h_kp1_k = std::sqrt(hv[m + 2 + k + 1]);
+            } else if (k >= 1 && k < (size_t)kMgsMax) {  // w = A z_k, then modified Gram-Schmidt in two passes
+                FX_TRY((launch_pt<T, 0>(ctx, RR, CC, Ld1<T>{Z[k]}, PtGmAv<T, MODE, false>{A, w, nullptr}, NoFin{},
+                                           nullptr, "fgmres_av")));
+                FX_TRY(mgs_two_pass(s, n, w, V, k + 1, dh));
+                FX_TRY(read_h(k));
+                for (size_t j = 0; j <= k; j++) H(j, k) = s->h_h[j];
+                h_kp1_k = std::sqrt(s->h_h[k + 1]);
             } else {
                 // w = A z_k with w.v_0, then modified Gram-Schmidt with each dot fused into the AXPY
                 FX_TRY((launch_pt<T, 1>(ctx, RR, CC, Ld1<T>{Z[k]}, PtGmAv<T, MODE, true>{A, w, V[0]}, FinSlot{dh + 0},
@@ -3804,7 +4058,7 @@ int fx_gmres_create(fx_ctx *ctx, const fx_grid *g, size_t restart, double tol, s
     s->grs.assign(restart + 1, 0.0);
     if (cudaMalloc(&s->d_h, (restart + 2) * sizeof(double)) != cudaSuccess ||
         cudaHostAlloc(&s->h_h, 2 * (restart + 2) * sizeof(double), cudaHostAllocMapped) != cudaSuccess ||
-        cudaHostGetDevicePointer((void **)&s->h_h_dev, s->h_h, 0) != cudaSuccess) {
+        cudaHostGetDevicePointer((void **)&s->h_h_dev, s->h_h, 0) != cudaSuccess || mgs_alloc(s) != FX_OK) {
         delete s;
         *out = nullptr;
         return fail(FX_ERR_BACKEND, "gmres scratch allocation failed");
@@ -3893,7 +4147,7 @@ int fx_fgmres_create(fx_ctx *ctx, const fx_grid *g, size_t restart, double tol, 
     s->grs.assign(restart + 1, 0.0);
     if (cudaMalloc(&s->d_h, (restart + 2) * sizeof(double)) != cudaSuccess ||
         cudaHostAlloc(&s->h_h, 2 * (restart + 2) * sizeof(double), cudaHostAllocMapped) != cudaSuccess ||
-        cudaHostGetDevicePointer((void **)&s->h_h_dev, s->h_h, 0) != cudaSuccess) {
+        cudaHostGetDevicePointer((void **)&s->h_h_dev, s->h_h, 0) != cudaSuccess || mgs_alloc(s) != FX_OK) {
         delete s;
         *out = nullptr;
         return fail(FX_ERR_BACKEND, "fgmres scratch allocation failed");
