@@ -416,6 +416,13 @@ class CudaBackend:
                                                C.byref(rr), C.byref(rw)))
         return rr.value, rw.value
 
+    def diffusion_steps(self, u, scratch, grid: Grid, stencil: Stencil, alpha: float, dt: float, scheme: int, n: int):
+        """`n` explicit diffusion steps on u (fx_diffusion_steps); scheme 0 Euler, 1 Heun, 2 RK4."""
+        s = StencilC(stencil)
+        g = grid_c(grid)
+        check(L.lib().fx_diffusion_steps(self.ctx, u.handle, scratch.handle, C.byref(g), s.ptr, float(alpha), float(dt),
+                                         int(scheme), int(n)))
+
     # -------------------------------------------------------------- vertex multigrid primitives
 
     @staticmethod

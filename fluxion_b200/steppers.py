@@ -239,7 +239,8 @@ class TimeScheme(enum.Enum):
 
 class DiffusionSolver:
     """solver.rs:30-642: explicit du/dt = alpha Lap u (+ source) by forward Euler, Heun (RK2) or
-    classical RK4, each stage the reference's sequence of field operations.  The default dt is
+    classical RK4, each stage the reference's sequence of field operations (in fused passes for zero
+    Dirichlet sides and no source, with the same values).  The default dt is
     the reference's stability bound safety * h_min^2 / (4 alpha) (safety 0.4 / 0.8 / 1.4).
     ``enable_graph()`` is the HipGraph path (solver.rs:182-325) on CUDA graphs: the first
     ``step_n`` records one step on the backend's stream and later steps replay it."""
@@ -290,7 +291,20 @@ class DiffusionSolver:
         """solver.rs:182-186 (enable_hip_graph)."""
         self._use_graph = True
 
+    def _fused(self, u: Field, n: int) -> bool:
+        """`n` steps without a source in the library's fused passes, where these hold: zero Dirichlet
+        sides, F64 (fx_diffusion_steps; the same values as the sequence of field operations)."""
+        if n < 1 or not self.boundaries.is_zero_dirichlet() or u.dtype() != DType.F64 or u.grid() != self.grid:
+            return False
+        u._same(self.scratch[0])
+        self.device.backend().diffusion_steps(u.storage, self.scratch[0].storage, self.grid, self.stencil, self.alpha,
+                                              self._dt, self._scheme.value, n)
+        self._steps_done += n
+        return True
+
     def step(self, u: Field, source: Optional[Field] = None) -> None:
+        if source is None and self._fused(u, 1):
+            return
         self._record(u, source)
         self._steps_done += 1
 
@@ -299,8 +313,14 @@ class DiffusionSolver:
         (one graph per solver, recorded on the first field passed)."""
         if n == 0:
             return
+        if not self._use_graph and self._fused(u, n):
+            return
         if self._use_graph:
-            if self._graph is None:
+            # the fused passes need no recording; the solver stays with the first field all the same
+            if self._graph is None and self._graph_u in (None, u) and self._fused(u, n):
+                self._graph_u = u
+                return
+            if self._graph is None and self._graph_u is None:
                 be = self.device.backend()
                 be.graph_begin()
                 try:

@@ -262,6 +262,13 @@ int fx_pcg_fused_update_dot2(fx_ctx *ctx, double alpha, double beta, fx_buf *z, 
                              fx_buf *p, fx_buf *x, fx_buf *r, fx_buf *w, const fx_buf *q,
                              double *rr, double *rw);
 
+/* `nsteps` explicit steps of du/dt = alpha Lap u (solver.rs:344-495) on u with homogeneous Dirichlet
+ * sides: scheme 0 forward Euler, 1 Heun (RK2), 2 classical RK4; s the five-point Laplacian.  The
+ * result equals the reference's sequence of field operations bit for bit; u and scratch (a field of
+ * the same grid, overwritten) are F64. */
+int fx_diffusion_steps(fx_ctx *ctx, fx_buf *u, fx_buf *scratch, const fx_grid *g, const fx_stencil *s, double alpha,
+                       double dt, int scheme, size_t nsteps);
+
 /* ------------------------------------------------------------------ */
 /* Vertex-centred multigrid primitives (full weighting, bilinear prolongation, true weighted
  * Jacobi).  Grids are (2^k+1) x (2^k+1)-style: fine = 2*(coarse-1)+1 in each direction.
