@@ -5,10 +5,18 @@
 //
 // Training runs on the CUDA cores in FP32 with the network's own rounding: weights and hidden
 // activations rounded to BF16 exactly as the tensor-core inference kernel rounds them, so a
-// trained network computes in training what it computes when applied.  Each block takes whole
-// samples; a thread owns a fixed set of parameters and accumulates their gradient over the
-// block's samples in registers, and one reduction kernel adds the blocks' partials in block
-// order, so a gradient is bitwise reproducible.
+// trained network computes in training what it computes when applied.  A block takes whole samples
+// and one reduction kernel adds the blocks' partial gradients in block order, so a gradient is
+// bitwise reproducible.
+//
+// A sample is 3.9 million fused multiply-adds, which the FP32 units bound (a block's operands stay in
+// shared memory); a thread computing one output, or one parameter's gradient, at a time loads two
+// operands for each and ran at 0.09 of the FP32 rate (2.43 ms for 2048 samples).  So every phase
+// is tiled in registers: the convolutions compute 8 (or 7) points of a row x 4 channels per thread,
+// the weight gradients 8 output channels x 3 taps of a row per thread over a share of the rows.
+// Activations lie point by point with their channels adjacent, padded so that the lanes of a warp
+// (4 channel groups x 8 rows, or 16 channels) fall in distinct banks: 0.55 ms, 0.40 of the FP32 rate,
+// with 18 warps per SM and the gradient sums spilled between phases.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -21,19 +29,30 @@ using namespace fx::lsm;
 
 namespace {
 
-constexpr int kTrThreads = 256;
-constexpr int kOwn = (kNParams + kTrThreads - 1) / kTrThreads;  // parameters per thread (12)
+constexpr int kTrThreads = 288;
 constexpr int kMaxPartBlocks = 1024;
 
 // shared-memory layout of the training kernel (floats)
-constexpr int kSmIn = kIn * kPin * kPin;   // 1875
-constexpr int kSmA1 = kC * kP1 * kP1;      // 8464: a1, later the gradient at a1's pre-activation
-constexpr int kSmA2 = kC * kP2 * kP2;      // 7056: a2, later the gradient at a2's pre-activation
-constexpr int kSmC = kP3 * kP3;            // 361: network output c, later dL/dc
-constexpr int kSmG = kT * kT;              // 256: dL/d(Hc), then 256: the whole-error part of dL/dc
-constexpr int kSmR = kNCo * kNCo;          // 81: R c, later P^T dL/d(Hc)
-constexpr int kSmW = kNParams;             // parameters (weights BF16-rounded)
-constexpr int kSmTrain = (kSmIn + kSmA1 + kSmA2 + 2 * kSmC + 2 * kSmG + kSmR + kSmW + 32) * 4;
+constexpr int kStr1 = 18;                      // a1: floats per point (16 channels; 8-byte aligned groups)
+constexpr int kStr2 = 20;                      // a2: floats per point (16-byte aligned groups)
+constexpr int kPad2 = kP2 + 4;                 // a2: points per row, two zero columns on each side
+constexpr int kSmA1 = kP1 * kP1 * kStr1;       // a1, later the gradient at a1's pre-activation
+constexpr int kSmA2 = kP2 * kPad2 * kStr2;     // a2, later the gradient at a2's pre-activation
+constexpr int kSmC = kP3 * kP3;                // 361: network output c; and as many: dL/dc
+constexpr int kSmG = kT * kT;                  // 256: dL/d(Hc), then 256: the whole-error part of dL/dc
+constexpr int kSmR = kNCo * kNCo;              // 81: R c, later P^T dL/d(Hc)
+constexpr int kSmW1 = kIn * 9 * kC;            // [ci][tap][co]
+constexpr int kSmW2 = kC * 9 * kC;             // [ci][tap][co], and as many [co][tap][ci]
+constexpr int kSmW3 = 9 * kC;                  // [tap][ci]
+constexpr int kSmInHalf = (kInLen + 5) / 2;    // BF16 inputs, and what the last row's tile reads past them
+constexpr int kSmTrainWords = kSmA1 + kSmA2 + kSmW1 + 2 * kSmW2 + kSmW3 + 2 * kC + 4 + 2 * (kSmC + 3) + 2 * kSmG +
+                              (kSmR + 3) + 32 + kSmInHalf;
+constexpr int kSmTrain = kSmTrainWords * 4;
+static_assert(2 * (kSmTrain + 1024) <= 228 * 1024, "two blocks per SM");
+// parts of the block that share a parameter's gradient: rows of the layer's output
+constexpr int kRg1 = 16, kRg2 = 3, kRg3 = 6, kRgB = kTrThreads / kC;
+static_assert(kRg2 * kSmW2 + kRg1 * kSmW1 + kRg3 * kSmW3 + 2 * kTrThreads + kTrThreads <= kSmA1 + kSmA2,
+              "the final sums fit the activations' space");
 
 // R at coarse point (I, J) of a field over the output region [-1, 17]^2 (index offset 1)
 __device__ __forceinline__ float fw19(const float *f, int I, int J) {
@@ -55,30 +74,61 @@ __device__ __forceinline__ float bil9(const float *Rc, int py, int px) {
     return 0.25f * ((r[0] + r[kNCo]) + (r[1] + r[kNCo + 1]));
 }
 
-// One block per group of samples: forward, loss and backward of each, gradients accumulated per
-// owned parameter; writes part[block][p] and part[block][kNParams] = the block's summed loss.
-__global__ void __launch_bounds__(kTrThreads) k_lsm_train(const float *__restrict__ wq,
-                                                          const __nv_bfloat16 *__restrict__ in_all,
-                                                          const float *__restrict__ tgt_all,
-                                                          const float *__restrict__ norm_all,
-                                                          const int *__restrict__ idx, int count, float lambda,
-                                                          float *__restrict__ part) {
+// One block per group of samples: forward, loss and backward of each, gradients accumulated in
+// registers over the block's samples; writes part[block][p] and part[block][kNParams] = the block's
+// summed loss.
+__global__ void __launch_bounds__(kTrThreads, 2) k_lsm_train(const float *__restrict__ wq,
+                                                             const __nv_bfloat16 *__restrict__ in_all,
+                                                             const float *__restrict__ tgt_all,
+                                                             const float *__restrict__ norm_all,
+                                                             const int *__restrict__ idx, int count, float lambda,
+                                                             float *__restrict__ part) {
     extern __shared__ __align__(16) float tsm[];
-    float *S_in = tsm;
-    float *S_a1 = S_in + kSmIn;
-    float *S_a2 = S_a1 + kSmA1;
-    float *S_c = S_a2 + kSmA2;
-    float *S_gc = S_c + kSmC;
-    float *S_gh = S_gc + kSmC;
+    float *S_a2 = tsm;  // 16-byte aligned groups first
+    float *S_w1 = S_a2 + kSmA2;
+    float *S_w2f = S_w1 + kSmW1;  // [ci][tap][co]
+    float *S_w2b = S_w2f + kSmW2;  // [co][tap][ci]
+    float *S_w3 = S_w2b + kSmW2;
+    float *S_b1 = S_w3 + kSmW3;
+    float *S_b2 = S_b1 + kC;
+    float *S_b3 = S_b2 + kC;
+    float *S_a1 = S_b3 + 4;
+    float *S_c = S_a1 + kSmA1;
+    float *S_gc = S_c + kSmC + 3;
+    float *S_gh = S_gc + kSmC + 3;
     float *S_ge = S_gh + kSmG;
     float *S_r = S_ge + kSmG;
-    float *S_w = S_r + kSmR;
-    float *S_red = S_w + kSmW;
+    float *S_red = S_r + kSmR + 3;
+    __nv_bfloat16 *S_in = reinterpret_cast<__nv_bfloat16 *>(S_red + 32);
     const int tid = threadIdx.x;
-    for (int p = tid; p < kNParams; p += kTrThreads) S_w[p] = wq[p];
-    float gacc[kOwn];
-#pragma unroll
-    for (int j = 0; j < kOwn; j++) gacc[j] = 0.f;
+    for (int p = tid; p < kSmW1; p += kTrThreads) {
+        const int co = p % kC, t = p / kC;
+        S_w1[p] = wq[w1(co, t / 9, t % 9)];
+    }
+    for (int p = tid; p < kSmW2; p += kTrThreads) {
+        const int lo = p % kC, t = p / kC;
+        S_w2f[p] = wq[w2(lo, t / 9, t % 9)];
+        S_w2b[p] = wq[w2(t / 9, lo, t % 9)];
+    }
+    for (int p = tid; p < kSmW3; p += kTrThreads) S_w3[p] = wq[w3(p % kC, p / kC)];
+    if (tid < kC) {
+        S_b1[tid] = wq[kOffB1 + tid];
+        S_b2[tid] = wq[kOffB2 + tid];
+    }
+    if (tid == 0) S_b3[0] = wq[kOffB3];
+    for (int p = tid; p < kSmA2; p += kTrThreads) S_a2[p] = 0.f;  // the zero columns stay zero
+    for (int p = tid; p < 2 * kSmInHalf; p += kTrThreads) S_in[p] = __float2bfloat16_rn(0.f);
+
+    // tiles of the convolutions: 4 channels (cg) of 8 or 7 points of a row
+    const int cg = tid & 3, trow1 = (tid >> 2) % kP1, tx1 = (tid >> 2) / kP1 * 8;
+    const int trow2 = (tid >> 2) % kP2, tx2 = (tid >> 2) / kP2 * 7;
+    const bool on1 = tid < 4 * kP1 * 3, on2 = tid < 4 * kP2 * 3;
+    // tiles of the weight gradients: 8 output channels x 3 taps of filter row ky, one input channel
+    const int g2ci = tid % kC, g2ky = tid / kC % 3, g2h = tid / 48 % 2, g2r = tid / 96;
+    const int g1t = tid % 18, g1ci = g1t % 3, g1ky = g1t / 3 % 3, g1h = g1t / 9, g1r = tid / 18;
+    const int g3ci = tid % kC, g3ky = tid / kC % 3, g3r = tid / 48;
+    const int bco = tid % kC, bgr = tid / kC;
+    float acc2[8][3] = {}, acc1[8][3] = {}, acc3[3] = {}, accb1 = 0.f, accb2 = 0.f, accb3 = 0.f;
     float loss_acc = 0.f;
     __syncthreads();
 
@@ -88,40 +138,95 @@ __global__ void __launch_bounds__(kTrThreads) k_lsm_train(const float *__restric
         const float *tgt = tgt_all + (size_t)s * kTgtLen;  // tH [256], tE [256]
         const float nrm = norm_all[2 * s] + lambda * norm_all[2 * s + 1];
         const float inv_n = nrm > 0.f ? 1.f / nrm : 0.f;
-        for (int k = tid; k < kSmIn; k += kTrThreads) S_in[k] = __bfloat162float(in[k]);
+        for (int k = tid; k < kInLen; k += kTrThreads) S_in[k] = in[k];
         __syncthreads();
-        // ---- forward
-        for (int o = tid; o < kC * kP1 * kP1; o += kTrThreads) {  // a1 = bf16(relu(conv1 + b1))
-            const int co = o / (kP1 * kP1), pix = o - co * (kP1 * kP1);
-            const int y = pix / kP1, x = pix - y * kP1;
-            float z = S_w[kOffB1 + co];
+        // ---- forward: every output accumulates over (ci, tap) from its bias
+        if (on1) {  // a1 = bf16(relu(conv1 + b1))
+            float z[8][4];
+#pragma unroll
+            for (int p = 0; p < 8; p++)
+#pragma unroll
+                for (int c = 0; c < 4; c++) z[p][c] = S_b1[cg * 4 + c];
+#pragma unroll
             for (int ci = 0; ci < kIn; ci++)
 #pragma unroll
-                for (int tap = 0; tap < 9; tap++)
-                    z = fmaf(S_w[w1(co, ci, tap)], S_in[ci * kPin * kPin + (y + tap / 3) * kPin + x + tap % 3], z);
-            S_a1[o] = bf16r(fmaxf(z, 0.f));
+                for (int ky = 0; ky < 3; ky++) {
+                    const __nv_bfloat16 *a = S_in + ci * kPin * kPin + (trow1 + ky) * kPin + tx1;
+                    float v[10];
+#pragma unroll
+                    for (int j = 0; j < 10; j++) v[j] = __bfloat162float(a[j]);
+#pragma unroll
+                    for (int kx = 0; kx < 3; kx++) {
+                        const float4 w = *reinterpret_cast<const float4 *>(S_w1 + (ci * 9 + ky * 3 + kx) * kC + cg * 4);
+#pragma unroll
+                        for (int p = 0; p < 8; p++) {
+                            z[p][0] = fmaf(w.x, v[p + kx], z[p][0]);
+                            z[p][1] = fmaf(w.y, v[p + kx], z[p][1]);
+                            z[p][2] = fmaf(w.z, v[p + kx], z[p][2]);
+                            z[p][3] = fmaf(w.w, v[p + kx], z[p][3]);
+                        }
+                    }
+                }
+#pragma unroll
+            for (int p = 0; p < 8; p++)
+                if (tx1 + p < kP1) {
+                    float2 *o = reinterpret_cast<float2 *>(S_a1 + (trow1 * kP1 + tx1 + p) * kStr1 + cg * 4);
+                    o[0] = make_float2(bf16r(fmaxf(z[p][0], 0.f)), bf16r(fmaxf(z[p][1], 0.f)));
+                    o[1] = make_float2(bf16r(fmaxf(z[p][2], 0.f)), bf16r(fmaxf(z[p][3], 0.f)));
+                }
         }
         __syncthreads();
-        for (int o = tid; o < kC * kP2 * kP2; o += kTrThreads) {  // a2 = bf16(relu(conv2 + b2))
-            const int co = o / (kP2 * kP2), pix = o - co * (kP2 * kP2);
-            const int y = pix / kP2, x = pix - y * kP2;
-            float z = S_w[kOffB2 + co];
-            for (int ci = 0; ci < kC; ci++) {
-                const float *a = S_a1 + ci * kP1 * kP1 + y * kP1 + x;
-                const float *w = S_w + w2(co, ci, 0);
+        if (on2) {  // a2 = bf16(relu(conv2 + b2))
+            float z[7][4];
 #pragma unroll
-                for (int tap = 0; tap < 9; tap++) z = fmaf(w[tap], a[(tap / 3) * kP1 + tap % 3], z);
-            }
-            S_a2[o] = bf16r(fmaxf(z, 0.f));
+            for (int p = 0; p < 7; p++)
+#pragma unroll
+                for (int c = 0; c < 4; c++) z[p][c] = S_b2[cg * 4 + c];
+#pragma unroll 2
+            for (int ci = 0; ci < kC; ci++)
+#pragma unroll
+                for (int ky = 0; ky < 3; ky++) {
+                    const float *a = S_a1 + ((trow2 + ky) * kP1 + tx2) * kStr1 + ci;
+                    float v[9];
+#pragma unroll
+                    for (int j = 0; j < 9; j++) v[j] = a[j * kStr1];
+#pragma unroll
+                    for (int kx = 0; kx < 3; kx++) {
+                        const float4 w = *reinterpret_cast<const float4 *>(S_w2f + (ci * 9 + ky * 3 + kx) * kC + cg * 4);
+#pragma unroll
+                        for (int p = 0; p < 7; p++) {
+                            z[p][0] = fmaf(w.x, v[p + kx], z[p][0]);
+                            z[p][1] = fmaf(w.y, v[p + kx], z[p][1]);
+                            z[p][2] = fmaf(w.z, v[p + kx], z[p][2]);
+                            z[p][3] = fmaf(w.w, v[p + kx], z[p][3]);
+                        }
+                    }
+                }
+#pragma unroll
+            for (int p = 0; p < 7; p++)
+                *reinterpret_cast<float4 *>(S_a2 + (trow2 * kPad2 + tx2 + p + 2) * kStr2 + cg * 4) =
+                    make_float4(bf16r(fmaxf(z[p][0], 0.f)), bf16r(fmaxf(z[p][1], 0.f)), bf16r(fmaxf(z[p][2], 0.f)),
+                                bf16r(fmaxf(z[p][3], 0.f)));
         }
         __syncthreads();
         for (int o = tid; o < kP3 * kP3; o += kTrThreads) {  // c = conv3 + b3
             const int y = o / kP3, x = o - y * kP3;
-            float z = S_w[kOffB3];
-            for (int ci = 0; ci < kC; ci++) {
-                const float *a = S_a2 + ci * kP2 * kP2 + y * kP2 + x;
+            float z = S_b3[0];
+            for (int ci = 0; ci < kC; ci += 4) {
+                float4 a[9], w[9];
 #pragma unroll
-                for (int tap = 0; tap < 9; tap++) z = fmaf(S_w[w3(ci, tap)], a[(tap / 3) * kP2 + tap % 3], z);
+                for (int tap = 0; tap < 9; tap++) {
+                    a[tap] = *reinterpret_cast<const float4 *>(S_a2 + ((y + tap / 3) * kPad2 + x + tap % 3 + 2) * kStr2 + ci);
+                    w[tap] = *reinterpret_cast<const float4 *>(S_w3 + tap * kC + ci);
+                }
+#pragma unroll
+                for (int tap = 0; tap < 9; tap++) z = fmaf(w[tap].x, a[tap].x, z);
+#pragma unroll
+                for (int tap = 0; tap < 9; tap++) z = fmaf(w[tap].y, a[tap].y, z);
+#pragma unroll
+                for (int tap = 0; tap < 9; tap++) z = fmaf(w[tap].z, a[tap].z, z);
+#pragma unroll
+                for (int tap = 0; tap < 9; tap++) z = fmaf(w[tap].w, a[tap].w, z);
             }
             S_c[o] = z;
         }
@@ -140,7 +245,7 @@ __global__ void __launch_bounds__(kTrThreads) k_lsm_train(const float *__restric
             S_gh[o] = -2.f * u * inv_n;
             S_ge[o] = -2.f * lambda * w * inv_n;
         }
-        // block sum of lsum: warp shuffles, then the 8 warp partials (the barrier also publishes
+        // block sum of lsum: warp shuffles, then the warp partials (the barrier also publishes
         // S_gh and ends the previous sample's reads of S_red)
         for (int off = 16; off > 0; off >>= 1) lsum += __shfl_down_sync(0xffffffffu, lsum, off);
         __syncthreads();
@@ -178,103 +283,186 @@ __global__ void __launch_bounds__(kTrThreads) k_lsm_train(const float *__restric
                 }
             }
             S_gc[o] = g;
+            accb3 += g;  // db3
         }
         __syncthreads();
-        // ---- conv3: dW3, db3 (owned parameters), then dL/dz2 in place of a2
-#pragma unroll
-        for (int j = 0; j < kOwn; j++) {
-            const int p = tid + j * kTrThreads;
-            if (p < kOffW3 || p >= kNParams) continue;
-            float acc = 0.f;
-            if (p == kOffB3) {
-                for (int o = 0; o < kP3 * kP3; o++) acc += S_gc[o];
-            } else {
-                const int ci = (p - kOffW3) / 9, tap = (p - kOffW3) % 9;
-                const float *a = S_a2 + ci * kP2 * kP2 + (tap / 3) * kP2 + tap % 3;
-                for (int y = 0; y < kP3; y++)
-                    for (int x = 0; x < kP3; x++) acc = fmaf(S_gc[y * kP3 + x], a[y * kP2 + x], acc);
-            }
-            gacc[j] += acc;
-        }
-        __syncthreads();
-        for (int o = tid; o < kC * kP2 * kP2; o += kTrThreads) {
-            const int ci = o / (kP2 * kP2), pix = o - ci * (kP2 * kP2);
-            const int y = pix / kP2, x = pix - y * kP2;
-            float g = 0.f;
-            if (S_a2[o] > 0.f) {
-#pragma unroll
-                for (int tap = 0; tap < 9; tap++) {
-                    const int cy = y - tap / 3, cx = x - tap % 3;
-                    if (cy < 0 || cx < 0 || cy >= kP3 || cx >= kP3) continue;
-                    g = fmaf(S_w[w3(ci, tap)], S_gc[cy * kP3 + cx], g);
+        // ---- conv3: dW3, then dL/dz2 in place of a2
+        {
+            float t[3] = {};
+            for (int y = g3r; y < kP3; y += kRg3) {
+                const float *a = S_a2 + ((y + g3ky) * kPad2 + 2) * kStr2 + g3ci;
+                float a0 = a[0], a1 = a[kStr2];
+#pragma unroll 4
+                for (int x = 0; x < kP3; x++) {
+                    const float a2 = a[(x + 2) * kStr2], g = S_gc[y * kP3 + x];
+                    t[0] = fmaf(g, a0, t[0]);
+                    t[1] = fmaf(g, a1, t[1]);
+                    t[2] = fmaf(g, a2, t[2]);
+                    a0 = a1;
+                    a1 = a2;
                 }
             }
-            S_a2[o] = g;  // dL/dz2 (ReLU mask from a2 itself)
+#pragma unroll
+            for (int k = 0; k < 3; k++) acc3[k] += t[k];
+        }
+        __syncthreads();
+        for (int o = tid; o < kP2 * kP2; o += kTrThreads) {
+            const int y = o / kP2, x = o - y * kP2;
+            float g[9];
+#pragma unroll
+            for (int tap = 0; tap < 9; tap++) {
+                const int cy = y - tap / 3, cx = x - tap % 3;
+                g[tap] = (cy < 0 || cx < 0 || cy >= kP3 || cx >= kP3) ? 0.f : S_gc[cy * kP3 + cx];
+            }
+            float4 *a = reinterpret_cast<float4 *>(S_a2 + (y * kPad2 + x + 2) * kStr2);
+#pragma unroll
+            for (int q = 0; q < kC / 4; q++) {
+                float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                for (int tap = 0; tap < 9; tap++) {
+                    const float4 w = *reinterpret_cast<const float4 *>(S_w3 + tap * kC + 4 * q);
+                    z.x = fmaf(w.x, g[tap], z.x);
+                    z.y = fmaf(w.y, g[tap], z.y);
+                    z.z = fmaf(w.z, g[tap], z.z);
+                    z.w = fmaf(w.w, g[tap], z.w);
+                }
+                const float4 v = a[q];  // ReLU mask from a2 itself
+                a[q] = make_float4(v.x > 0.f ? z.x : 0.f, v.y > 0.f ? z.y : 0.f, v.z > 0.f ? z.z : 0.f,
+                                   v.w > 0.f ? z.w : 0.f);
+            }
         }
         __syncthreads();
         // ---- conv2: dW2, db2, then dL/dz1 in place of a1
+        {
+            float t[8][3] = {};
+            for (int y = 7 * g2r; y < 7 * g2r + 7; y++) {
+                const float *a = S_a1 + (y + g2ky) * kP1 * kStr1 + g2ci;
+                const float *gz = S_a2 + (y * kPad2 + 2) * kStr2 + 8 * g2h;
+                float a0 = a[0], a1 = a[kStr1];
+#pragma unroll 3
+                for (int x = 0; x < kP2; x++) {
+                    const float a2 = a[(x + 2) * kStr1];
+                    const float4 lo = *reinterpret_cast<const float4 *>(gz + x * kStr2);
+                    const float4 hi = *reinterpret_cast<const float4 *>(gz + x * kStr2 + 4);
+                    const float g[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
 #pragma unroll
-        for (int j = 0; j < kOwn; j++) {
-            const int p = tid + j * kTrThreads;
-            if (p < kOffW2 || p >= kOffW3) continue;
-            float acc = 0.f;
-            if (p >= kOffB2) {
-                const float *g = S_a2 + (p - kOffB2) * kP2 * kP2;
-                for (int o = 0; o < kP2 * kP2; o++) acc += g[o];
-            } else {
-                const int co = (p - kOffW2) / (kC * 9), ci = ((p - kOffW2) / 9) % kC, tap = (p - kOffW2) % 9;
-                const float *g = S_a2 + co * kP2 * kP2;
-                const float *a = S_a1 + ci * kP1 * kP1 + (tap / 3) * kP1 + tap % 3;
-                for (int y = 0; y < kP2; y++)
-                    for (int x = 0; x < kP2; x++) acc = fmaf(g[y * kP2 + x], a[y * kP1 + x], acc);
-            }
-            gacc[j] += acc;
-        }
-        __syncthreads();
-        for (int o = tid; o < kC * kP1 * kP1; o += kTrThreads) {
-            const int ci = o / (kP1 * kP1), pix = o - ci * (kP1 * kP1);
-            const int y = pix / kP1, x = pix - y * kP1;
-            float g = 0.f;
-            if (S_a1[o] > 0.f) {
-                for (int co = 0; co < kC; co++) {
-                    const float *gz = S_a2 + co * kP2 * kP2;
-                    const float *w = S_w + w2(co, ci, 0);
-#pragma unroll
-                    for (int tap = 0; tap < 9; tap++) {
-                        const int zy = y - tap / 3, zx = x - tap % 3;
-                        if (zy < 0 || zx < 0 || zy >= kP2 || zx >= kP2) continue;
-                        g = fmaf(w[tap], gz[zy * kP2 + zx], g);
+                    for (int c = 0; c < 8; c++) {
+                        t[c][0] = fmaf(g[c], a0, t[c][0]);
+                        t[c][1] = fmaf(g[c], a1, t[c][1]);
+                        t[c][2] = fmaf(g[c], a2, t[c][2]);
                     }
+                    a0 = a1;
+                    a1 = a2;
                 }
             }
-            S_a1[o] = g;  // dL/dz1
+#pragma unroll
+            for (int c = 0; c < 8; c++)
+#pragma unroll
+                for (int k = 0; k < 3; k++) acc2[c][k] += t[c][k];
+            float b = 0.f;
+            for (int o = bgr; o < kP2 * kP2; o += kRgB) b += S_a2[(o / kP2 * kPad2 + o % kP2 + 2) * kStr2 + bco];
+            accb2 += b;
+        }
+        __syncthreads();
+        if (on1) {  // dL/dz1 of 4 input channels (cg) of 8 points: transposed filters over the padded rows
+            float z[8][4] = {};
+#pragma unroll 2
+            for (int co = 0; co < kC; co++)
+#pragma unroll
+                for (int ky = 0; ky < 3; ky++) {
+                    const int zy = trow1 - ky;
+                    if (zy < 0 || zy >= kP2) continue;
+                    const float *gz = S_a2 + (zy * kPad2 + tx1) * kStr2 + co;
+                    float v[10];
+#pragma unroll
+                    for (int j = 0; j < 10; j++) v[j] = gz[j * kStr2];  // v[j]: point tx1 + j - 2
+#pragma unroll
+                    for (int kx = 0; kx < 3; kx++) {
+                        const float4 w = *reinterpret_cast<const float4 *>(S_w2b + (co * 9 + ky * 3 + kx) * kC + cg * 4);
+#pragma unroll
+                        for (int p = 0; p < 8; p++) {
+                            z[p][0] = fmaf(w.x, v[p + 2 - kx], z[p][0]);
+                            z[p][1] = fmaf(w.y, v[p + 2 - kx], z[p][1]);
+                            z[p][2] = fmaf(w.z, v[p + 2 - kx], z[p][2]);
+                            z[p][3] = fmaf(w.w, v[p + 2 - kx], z[p][3]);
+                        }
+                    }
+                }
+#pragma unroll
+            for (int p = 0; p < 8; p++)
+                if (tx1 + p < kP1) {
+                    float2 *o = reinterpret_cast<float2 *>(S_a1 + (trow1 * kP1 + tx1 + p) * kStr1 + cg * 4);
+                    const float2 u = o[0], v = o[1];
+                    o[0] = make_float2(u.x > 0.f ? z[p][0] : 0.f, u.y > 0.f ? z[p][1] : 0.f);
+                    o[1] = make_float2(v.x > 0.f ? z[p][2] : 0.f, v.y > 0.f ? z[p][3] : 0.f);
+                }
         }
         __syncthreads();
         // ---- conv1: dW1, db1
+        {
+            float t[8][3] = {};
+            for (int y = g1r; y < kP1; y += kRg1) {
+                const __nv_bfloat16 *a = S_in + g1ci * kPin * kPin + (y + g1ky) * kPin;
+                const float *gz = S_a1 + y * kP1 * kStr1 + 8 * g1h;
+                float a0 = __bfloat162float(a[0]), a1 = __bfloat162float(a[1]);
+                for (int x = 0; x < kP1; x++) {
+                    const float a2 = __bfloat162float(a[x + 2]);
+                    const float2 *gp = reinterpret_cast<const float2 *>(gz + x * kStr1);
+                    const float2 g01 = gp[0], g23 = gp[1], g45 = gp[2], g67 = gp[3];
+                    const float g[8] = {g01.x, g01.y, g23.x, g23.y, g45.x, g45.y, g67.x, g67.y};
 #pragma unroll
-        for (int j = 0; j < kOwn; j++) {
-            const int p = tid + j * kTrThreads;
-            if (p >= kOffW2) continue;
-            float acc = 0.f;
-            if (p >= kOffB1) {
-                const float *g = S_a1 + (p - kOffB1) * kP1 * kP1;
-                for (int o = 0; o < kP1 * kP1; o++) acc += g[o];
-            } else {
-                const int co = p / (kIn * 9), ci = (p / 9) % kIn, tap = p % 9;
-                const float *g = S_a1 + co * kP1 * kP1;
-                const float *a = S_in + ci * kPin * kPin + (tap / 3) * kPin + tap % 3;
-                for (int y = 0; y < kP1; y++)
-                    for (int x = 0; x < kP1; x++) acc = fmaf(g[y * kP1 + x], a[y * kPin + x], acc);
+                    for (int c = 0; c < 8; c++) {
+                        t[c][0] = fmaf(g[c], a0, t[c][0]);
+                        t[c][1] = fmaf(g[c], a1, t[c][1]);
+                        t[c][2] = fmaf(g[c], a2, t[c][2]);
+                    }
+                    a0 = a1;
+                    a1 = a2;
+                }
             }
-            gacc[j] += acc;
+#pragma unroll
+            for (int c = 0; c < 8; c++)
+#pragma unroll
+                for (int k = 0; k < 3; k++) acc1[c][k] += t[c][k];
+            float b = 0.f;
+            for (int o = bgr; o < kP1 * kP1; o += kRgB) b += S_a1[o * kStr1 + bco];
+            accb1 += b;
         }
         __syncthreads();
     }
-    float *out = part + (size_t)blockIdx.x * (kNParams + 1);
+    // ---- the parts of each parameter's gradient, added in a fixed order
+    float *T2 = tsm, *T1 = T2 + kRg2 * kSmW2, *T3 = T1 + kRg1 * kSmW1, *TB = T3 + kRg3 * kSmW3;
+    static_assert(kSmA2 + kSmW1 + 2 * kSmW2 + kSmW3 + 2 * kC + 4 + kSmA1 >=
+                      kRg2 * kSmW2 + kRg1 * kSmW1 + kRg3 * kSmW3 + 3 * kTrThreads, "final sums");
 #pragma unroll
-    for (int j = 0; j < kOwn; j++) {
-        const int p = tid + j * kTrThreads;
-        if (p < kNParams) out[p] = gacc[j];
+    for (int c = 0; c < 8; c++)
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            T2[g2r * kSmW2 + ((8 * g2h + c) * kC + g2ci) * 9 + 3 * g2ky + k] = acc2[c][k];
+            T1[g1r * kSmW1 + ((8 * g1h + c) * kIn + g1ci) * 9 + 3 * g1ky + k] = acc1[c][k];
+        }
+#pragma unroll
+    for (int k = 0; k < 3; k++) T3[g3r * kSmW3 + g3ci * 9 + 3 * g3ky + k] = acc3[k];
+    TB[tid] = accb1;
+    TB[kTrThreads + tid] = accb2;
+    TB[2 * kTrThreads + tid] = accb3;
+    __syncthreads();
+    float *out = part + (size_t)blockIdx.x * (kNParams + 1);
+    for (int p = tid; p < kNParams; p += kTrThreads) {
+        float g = 0.f;
+        if (p < kOffB1)
+            for (int r = 0; r < kRg1; r++) g += T1[r * kSmW1 + p - kOffW1];
+        else if (p < kOffW2)
+            for (int r = 0; r < kRgB; r++) g += TB[r * kC + p - kOffB1];
+        else if (p < kOffB2)
+            for (int r = 0; r < kRg2; r++) g += T2[r * kSmW2 + p - kOffW2];
+        else if (p < kOffW3)
+            for (int r = 0; r < kRgB; r++) g += TB[kTrThreads + r * kC + p - kOffB2];
+        else if (p < kOffB3)
+            for (int r = 0; r < kRg3; r++) g += T3[r * kSmW3 + p - kOffW3];
+        else
+            for (int r = 0; r < kTrThreads; r++) g += TB[2 * kTrThreads + r];
+        out[p] = g;
     }
     if (tid == 0) out[kNParams] = loss_acc;
 }
