@@ -329,12 +329,13 @@ int launch_rows(fx_ctx *ctx, size_t rows, size_t cols, F f, const char *what) {
     return check_launch(ctx, what);
 }
 
-// the iterate, corrected by the piecewise-constant prolongation of `e` when that is not null
+// the iterate (zero when u is null), corrected by the piecewise-constant prolongation of `e` when
+// that is not null
 struct ChebIn {
     const double *u, *e;
     int cols, ccols;
     __device__ __forceinline__ double at(int r, int c, size_t i) const {
-        const double v = u[i];
+        const double v = u ? u[i] : 0.0;
         return e ? v + e[(size_t)(r >> 1) * ccols + (c >> 1)] : v;
     }
     __device__ __forceinline__ Nb<double> nb(int r, int c, size_t i) const {
@@ -411,9 +412,186 @@ struct RefRestrict {
         const int fr = 2 * r, fc = 2 * c;
         const int fr1 = fr + 1 < rows - 1 ? fr + 1 : rows - 1, fc1 = fc + 1 < cols - 1 ? fc + 1 : cols - 1;
         crhs[i] = 0.25 * (((resid(fr, fc) + resid(fr1, fc)) + resid(fr, fc1)) + resid(fr1, fc1));
-        cu[i] = 0.0;
+        if (cu) cu[i] = 0.0;
     }
 };
+
+// ---------------------------------------------------------------- the Chebyshev hierarchy's tail
+//
+// The coarse levels in one block, every vector in shared memory.  A launch of a small level costs
+// 1.9 us whatever it computes, and a cycle from 64 x 48 down makes 34 of them; in one block a step
+// is a barrier, a shared round trip and the point's chain of ten dependent operations.  What then
+// bounds it is instruction issue and that chain, so: a level is worked on by the warps it has points
+// for and the others sleep at a barrier (all warps through every step: 36 us), the residual is taken
+// once per fine point and not four times around the average, and the ring's four sides share one
+// code path (those two: 32 -> 25 us).  MG-PCG on 1024 x 768, 33 cycles: 5.07 -> 3.96 ms.
+// A level's three iterates rotate: after n steps the iterate is buffer n mod 3, so nothing is copied.
+// The tail starts at the first level whose vectors, with those below it, fit in 200 KB (4800 points
+// or so); a larger level has work for more than one SM.
+
+constexpr int kChebTailLevels = 10;
+constexpr int kChebTailSteps = 32;
+constexpr int kChebTailThreads = 512;  // 1024: level
+constexpr size_t kChebTailSmem = 200 * 1024;
+
+struct ChebTailLevel {
+    int rows, cols;
+    unsigned magic;  // 2^32 / cols, rounded up: i / cols = umulhi(i, magic) for i * cols < 2^32
+    double w[5];     // centre, north, south, west, east
+    double f, inv_diag;
+    BcP B;
+};
+
+struct ChebTailArgs {
+    const double *u_in;  // null: zero
+    const double *rhs;
+    double *u_out;
+    int nlev, n_pre, n_post, n_coarse;
+    ChebTailLevel L[kChebTailLevels];
+    double os[kChebTailSteps], om[kChebTailSteps];  // of the steps after the first
+};
+
+__global__ void __launch_bounds__(kChebTailThreads) k_cheb_tail(const __grid_constant__ ChebTailArgs A_in) {
+    // the arguments in shared memory: read a level at a time they would miss the constant cache in
+    // every one of the short steps
+    __shared__ ChebTailArgs A;
+    static_assert(sizeof(ChebTailArgs) % sizeof(long long) == 0, "copied by words");
+    for (int i = threadIdx.x; i < (int)(sizeof(ChebTailArgs) / sizeof(long long)); i += blockDim.x)
+        reinterpret_cast<long long *>(&A)[i] = reinterpret_cast<const long long *>(&A_in)[i];
+    grid_dep_enter();
+    __syncthreads();
+    extern __shared__ double ct_smem[];  // level l: iterates 0, 1, 2 and the rhs, n values each
+    double *const sm = ct_smem;
+    // a level is worked on by as many warps as it has points for; the others wait at the barrier of
+    // the level above until the cycle comes back up (barrier 1 + l: level l's warps)
+    auto warps = [&](int l) { return min((int)blockDim.x >> 5, (A.L[l].rows * A.L[l].cols + 31) >> 5); };
+    auto sync = [](int l, int w) { asm volatile("barrier.sync %0, %1;" ::"r"(1 + l), "r"(w * 32) : "memory"); };
+    const int wid = threadIdx.x >> 5, last = A.nlev - 1;
+    {
+        const int n0 = A.L[0].rows * A.L[0].cols;
+        for (int i = threadIdx.x; i < n0; i += blockDim.x) {
+            sm[i] = A.u_in ? A.u_in[i] : 0.0;
+            sm[3 * n0 + i] = A.rhs[i];
+        }
+        __syncthreads();
+    }
+    int off = 0, e = 0;  // of the level; of the correction to add
+    int k = 0;           // the iterate
+    for (int v = 0; v <= 2 * last; v++) {  // down to the coarsest level and up again
+        const bool down = v < last;
+        const int l = v <= last ? v : 2 * last - v;
+        const ChebTailLevel &L = A.L[l];
+        const int rows = L.rows, cols = L.cols, np = rows * cols, nw = warps(l);
+        const unsigned magic = L.magic;
+        if (wid < nw) {
+            auto points = [&](int pc, int n, unsigned mg, auto f) {
+#pragma unroll 1
+                for (int i = threadIdx.x; i < n; i += nw * 32) {
+                    const int r = (int)__umulhi((unsigned)i, mg);
+                    f(r, i - r * pc, i);
+                }
+                sync(l, nw);
+            };
+            const double *const rhs = sm + (off + 3 * np);
+            const double wc = L.w[0], wn = L.w[1], ws = L.w[2], ww = L.w[3], we = L.w[4], f = L.f, inv_diag = L.inv_diag;
+            auto ring = [&](int r, int c) { return r == 0 || c == 0 || r == rows - 1 || c == cols - 1; };
+            auto apply = [&](const double *u) {  // stencil_eval<double, 5>
+                StencilP P;
+                P.c = wc, P.n = wn, P.s = ws, P.w = ww, P.e = we;
+                Nb<double> nb;
+                nb.c = u[0], nb.n = u[-cols], nb.s = u[cols], nb.w = u[-1], nb.e = u[1];
+                nb.nw = nb.ne = nb.sw = nb.se = 0.0;
+                return stencil_eval<double, 5>(P, nb);
+            };
+            const int n = down ? A.n_pre : (v == last ? A.n_coarse : A.n_post);
+            k = v <= last ? 0 : A.n_pre % 3;
+            if (v > last) {
+                sync(l, nw);  // the level below is done
+                const int cc = A.L[l + 1].cols, u = off + k * np;
+                points(cols, np, magic, [&](int r, int c, int i) { sm[u + i] += sm[e + (r >> 1) * cc + (c >> 1)]; });
+            }
+            for (int i = 0; i < n; i++) {  // ChebFirst, ChebNext
+                const int k1 = k == 2 ? 0 : k + 1, km = k == 0 ? 2 : k - 1;
+                const double *const u = sm + (off + k * np), *const um = sm + (off + km * np);
+                double *const out = sm + (off + k1 * np);
+                if (i == 0) {
+                    points(cols, np, magic, [&](int r, int c, int p) {
+                        out[p] = ring(r, c) ? 0.0 : fma(1.0, u[p], fma(-1.0, apply(u + p), rhs[p]) * f);
+                    });
+                } else {
+                    const double om = A.om[i], os = A.os[i], om1 = 1.0 - om;
+                    points(cols, np, magic, [&](int r, int c, int p) {
+                        double d = 0.0;
+                        if (!ring(r, c)) {
+                            d = fma(-1.0, apply(u + p), rhs[p]) * inv_diag;
+                            d = fma(om1, um[p], fma(om, u[p], d * os));
+                        }
+                        out[p] = d;
+                    });
+                }
+                k = k1;
+            }
+            if (down) {  // RefRestrict: the residual once per point into the free iterate, then the averages
+                const ChebTailLevel &C = A.L[l + 1];
+                const int nc = C.rows * C.cols, cc = C.cols;
+                const double *const u = sm + (off + k * np);
+                double *const res = sm + (off + (k == 2 ? 0 : k + 1) * np), *const cu = sm + (off + 4 * np);
+                points(cols, np, magic, [&](int r, int c, int p) {
+                    double t;
+                    if (ring(r, c)) {
+                        const int side = r == 0 ? 0 : (r == rows - 1 ? 1 : (c == 0 ? 2 : 3));
+                        const int d = side == 0 ? cols : (side == 1 ? -cols : (side == 2 ? 1 : -1));
+                        t = bc_value(L.B, side, u[p], u[p + d], side < 2 ? L.B.dy : L.B.dx);
+                    } else {
+                        t = apply(u + p);
+                    }
+                    res[p] = fma(1.0, rhs[p], t * -1.0);
+                });
+                points(cc, nc, C.magic, [&](int r, int c, int p) {
+                    const int fr1 = min(2 * r + 1, rows - 1), fc1 = min(2 * c + 1, cols - 1);
+                    const double *const r0 = res + 2 * r * cols, *const r1 = res + fr1 * cols;
+                    cu[3 * nc + p] = 0.25 * (((r0[2 * c] + r1[2 * c]) + r0[fc1]) + r1[fc1]);
+                    cu[p] = 0.0;
+                });
+            }
+        }
+        if (down) {
+            off += 4 * np;
+        } else if (l > 0) {
+            e = off + (v == last ? A.n_coarse : A.n_pre + A.n_post) % 3 * np;
+            off -= 4 * A.L[l - 1].rows * A.L[l - 1].cols;
+        }
+    }
+    const int n0 = A.L[0].rows * A.L[0].cols;
+    if (wid < warps(0))
+        for (int i = threadIdx.x; i < n0; i += warps(0) * 32) A.u_out[i] = sm[k * n0 + i];
+}
+
+// the Chebyshev recurrence over the fixed spectrum [0.2, 2] (multigrid.rs:308-473)
+struct ChebSeq {
+    double scale, mu, omegaprod, c_km1, c_k;
+    ChebSeq() {
+        const double emax = 2.0, emin = 0.1 * emax;
+        scale = 2.0 / (emax + emin);
+        const double alpha = 1.0 - scale * emin;
+        mu = 1.0 / alpha;
+        omegaprod = 2.0 / alpha;
+        c_km1 = 1.0;
+        c_k = mu;
+    }
+    double next() {  // omega of the next step
+        const double c_kp1 = 2.0 * mu * c_k - c_km1;
+        const double omega = omegaprod * c_k / c_kp1;
+        c_km1 = c_k;
+        c_k = c_kp1;
+        return omega;
+    }
+};
+
+double cheb_inv_diag(double dx, double dy) {
+    const double inv_dx2 = 1.0 / (dx * dx), inv_dy2 = 1.0 / (dy * dy);
+    return -1.0 / (2.0 * inv_dx2 + 2.0 * inv_dy2);
+}
 
 template <typename T, int NW>
 int lex5_launch(fx_ctx *ctx, const LexArgs<T> &A, int warps) {
@@ -489,23 +667,17 @@ template int lex5_sweeps<float>(fx_ctx *, float *, const float *, size_t, size_t
 template int lex5_sweeps<double>(fx_ctx *, double *, const double *, size_t, size_t, const double (&)[5], double, double,
                                  size_t);
 
-int cheb_smooth(fx_ctx *ctx, const ChebLevel &L, const double *coarse, size_t ccols, size_t n) {
+int cheb_smooth(fx_ctx *ctx, const ChebLevel &L, const double *coarse, size_t ccols, size_t n, bool u_zero) {
     if (n == 0) return FX_OK;
-    const double emax = 2.0, emin = 0.1 * emax;
-    const double scale = 2.0 / (emax + emin);
-    const double alpha = 1.0 - scale * emin;
-    const double mu = 1.0 / alpha, omegaprod = 2.0 / alpha;
-    const double inv_dx2 = 1.0 / (L.dx * L.dx), inv_dy2 = 1.0 / (L.dy * L.dy);
-    const double inv_diag = -1.0 / (2.0 * inv_dx2 + 2.0 * inv_dy2);
+    ChebSeq seq;
+    const double inv_diag = cheb_inv_diag(L.dx, L.dy), scale = seq.scale;
     const int rows = (int)L.rows, cols = (int)L.cols;
-    double c_km1 = 1.0, c_k = mu;
-    const ChebIn in{L.u, coarse, cols, (int)ccols};
+    const ChebIn in{u_zero ? nullptr : L.u, coarse, cols, (int)ccols};
     FX_TRY(launch_rows(ctx, L.rows, L.cols, ChebFirst{in, L.rhs, L.w0, L.P, scale * inv_diag, rows, cols}, "cheb_step"));
     double *buf[3] = {L.u, L.w0, L.w1};
     int km1 = 0, k = 1, kp1 = 2;
     for (size_t i = 1; i < n; i++) {
-        const double c_kp1 = 2.0 * mu * c_k - c_km1;
-        const double omega = omegaprod * c_k / c_kp1;
+        const double omega = seq.next();
         // the last step writes u itself where it may: x_{k-1} is read at the point alone, x_k around it
         double *out = i + 1 == n && k != 0 ? L.u : buf[kp1];
         const ChebIn prev = i == 1 ? in : ChebIn{buf[km1], nullptr, cols, 0};
@@ -513,8 +685,6 @@ int cheb_smooth(fx_ctx *ctx, const ChebLevel &L, const double *coarse, size_t cc
                            ChebNext{buf[k], prev, L.rhs, out, L.P, inv_diag, omega * scale, omega, 1.0 - omega, rows, cols},
                            "cheb_step"));
         if (i + 1 == n && out == L.u) return FX_OK;
-        c_km1 = c_k;
-        c_k = c_kp1;
         const int t = km1;
         km1 = k;
         k = kp1;
@@ -523,6 +693,59 @@ int cheb_smooth(fx_ctx *ctx, const ChebLevel &L, const double *coarse, size_t cc
     if (buf[k] != L.u)
         FX_CUDA(cudaMemcpyAsync(L.u, buf[k], L.rows * L.cols * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream));
     return FX_OK;
+}
+
+int cheb_tail_top(const ChebLevel *L, int nl, size_t n_pre, size_t n_post, size_t n_coarse) {
+    if (n_post == 0 || std::max(n_coarse, n_pre) > (size_t)kChebTailSteps) return nl;
+    int top = nl;
+    size_t bytes = 0;
+    for (int l = nl - 1; l >= 0 && nl - l <= kChebTailLevels; l--) {
+        // the prolongation onto this level stays inside the coarser one
+        if (l + 1 < nl && ((L[l].rows - 1) / 2 > L[l + 1].rows - 1 || (L[l].cols - 1) / 2 > L[l + 1].cols - 1)) break;
+        if (L[l].rows < 2 || L[l].cols < 2 || L[l].rows > kChebTailSmem || L[l].cols > kChebTailSmem) break;
+        bytes += 4 * sizeof(double) * L[l].rows * L[l].cols;
+        if (bytes > kChebTailSmem) break;
+        top = l;
+    }
+    return top;
+}
+
+int cheb_tail(fx_ctx *ctx, const ChebLevel *L, const BcP *B, int nlev, bool u_zero, size_t n_pre, size_t n_post,
+              size_t n_coarse) {
+    ChebTailArgs A;
+    A.u_in = u_zero ? nullptr : L[0].u;
+    A.rhs = L[0].rhs;
+    A.u_out = L[0].u;
+    A.nlev = nlev;
+    A.n_pre = (int)n_pre;
+    A.n_post = (int)n_post;
+    A.n_coarse = (int)n_coarse;
+    ChebSeq seq;
+    const double scale = seq.scale;
+    A.os[0] = A.om[0] = 0.0;
+    for (int i = 1; i < kChebTailSteps; i++) {
+        A.om[i] = seq.next();
+        A.os[i] = A.om[i] * scale;
+    }
+    size_t bytes = 0;
+    for (int l = 0; l < nlev; l++) {
+        ChebTailLevel &T = A.L[l];
+        T.rows = (int)L[l].rows;
+        T.cols = (int)L[l].cols;
+        T.magic = (unsigned)((1ull << 32) / L[l].cols + 1);
+        const StencilP &P = L[l].P;
+        T.w[0] = P.c, T.w[1] = P.n, T.w[2] = P.s, T.w[3] = P.w, T.w[4] = P.e;
+        T.inv_diag = cheb_inv_diag(L[l].dx, L[l].dy);
+        T.f = scale * T.inv_diag;
+        T.B = B[l];
+        bytes += 4 * sizeof(double) * L[l].rows * L[l].cols;
+    }
+    FX_TRY(strip_smem_optin(k_cheb_tail, kChebTailSmem));
+    const size_t n0 = L[0].rows * L[0].cols;
+    timing_pre(ctx, "cheb_tail");
+    launch_pdl(ctx, k_cheb_tail, dim3(1), dim3((unsigned)std::min<size_t>(kChebTailThreads, (n0 + 31) / 32 * 32)), bytes, A);
+    timing_post(ctx, (double)n0);
+    return check_launch(ctx, "cheb_tail");
 }
 
 int ref_restrict_residual(fx_ctx *ctx, const double *u, const double *rhs, size_t rows, size_t cols, const StencilP &P,

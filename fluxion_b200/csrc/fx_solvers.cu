@@ -338,6 +338,7 @@ struct fx_mg {
         int apply(fx_buf *z, const fx_buf *r, const int *skip, bool z_zero) override;
         int apply_pcg(fx_buf *z, const fx_buf *r, const int *skip, DevState *S, bool first) override;
         bool fills_from_zero(const fx_buf *z) const override;
+        bool writes_all() const override { return mg->mode == 0; }
     } view;
     ~fx_mg() {
         for (auto &L : lv) {
@@ -557,7 +558,8 @@ int convert(fx_ctx *ctx, const S *src, D *dst, size_t n, const int *skip) {
 // Reference-semantics cycle (multigrid.rs:188-230).  Each phase is the sequence of backend ops the
 // reference runs, fused where that leaves every value as it is (fx_reference.cu): consecutive
 // Jacobi sweeps in one launch, a Chebyshev step per launch (the first after a prolongation takes
-// the correction with it), residual and restriction in one.
+// the correction with it, the first of a zero iterate none), residual and restriction in one, and
+// under the Chebyshev smoother the levels of a few thousand points and below in one block.
 int reference_cycle(fx_mg *mg, fx_buf *x, const fx_buf *b, bool x_zero) {
     fx_ctx *ctx = mg->ctx;
     const int nl = (int)mg->lv.size();
@@ -579,10 +581,22 @@ int reference_cycle(fx_mg *mg, fx_buf *x, const fx_buf *b, bool x_zero) {
         FX_TRY(make_stencil(&s, &P[l]));
         if (nl > 1 || mg->smoother == 1) FX_TRY(make_bc(&mg->bc, mg->lv[l].dx, mg->lv[l].dy, &B[l], true));
     }
-    if (x_zero) FX_CUDA(cudaMemsetAsync(u_of(0), 0, L0.rows * L0.cols * sizeof(double), ctx->stream));
-    // smoothing on level l, after adding the prolongation of level l + 1's u when `correct`
-    auto smooth = [&](int l, size_t n, bool correct) -> int {
+    std::vector<ChebLevel> V;
+    int top = nl;  // the levels from here on run in one block
+    if (mg->smoother == 1) {
+        for (int l = 0; l < nl; l++) {
+            const MgLevel &L = mg->lv[l];
+            V.push_back({L.rows, L.cols, L.dx, L.dy, P[l], u_of(l), (double *)L.w0->ptr, (double *)L.w1->ptr, rhs_of(l)});
+        }
+        top = cheb_tail_top(V.data(), nl, mg->n_pre, mg->n_post, mg->n_pre + mg->n_post + 10);
+    }
+    // whether level l's first smoothing takes its zero iterate as such instead of reading it
+    auto zero_first = [&](int l) { return mg->smoother == 1 && (l >= top || mg->n_pre > 0 || l == nl - 1); };
+    if (x_zero && !zero_first(0)) FX_CUDA(cudaMemsetAsync(u_of(0), 0, L0.rows * L0.cols * sizeof(double), ctx->stream));
+    // level l's first smoothing, or the one that follows the prolongation of level l + 1's u
+    auto smooth = [&](int l, size_t n, bool first) -> int {
         MgLevel &L = mg->lv[l];
+        bool correct = !first;
         if (correct) {
             MgLevel &C = mg->lv[l + 1];
             const fx_grid g{L.rows, L.cols, L.dx, L.dy}, cg{C.rows, C.cols, C.dx, C.dy};
@@ -598,21 +612,23 @@ int reference_cycle(fx_mg *mg, fx_buf *x, const fx_buf *b, bool x_zero) {
                 correct = false;
             }
         }
-        if (mg->smoother == 1) {
-            const ChebLevel V{L.rows, L.cols, L.dx, L.dy, P[l], u_of(l), (double *)L.w0->ptr, (double *)L.w1->ptr, rhs_of(l)};
-            return cheb_smooth(ctx, V, correct ? (const double *)mg->lv[l + 1].u->ptr : nullptr,
-                               correct ? mg->lv[l + 1].cols : 0, n);
-        }
+        if (mg->smoother == 1)
+            return cheb_smooth(ctx, V[l], correct ? (const double *)mg->lv[l + 1].u->ptr : nullptr,
+                               correct ? mg->lv[l + 1].cols : 0, n, first && (l > 0 || x_zero) && zero_first(l));
         return lex5_sweeps<double>(ctx, u_of(l), rhs_of(l), L.rows, L.cols, L.lap5, mg->omega, 1.0 / L.lap5[0], n);
     };
-    for (int l = 0; l < nl - 1; l++) {
+    const size_t n_coarse = mg->n_pre + mg->n_post + 10;
+    for (int l = 0; l < nl - 1 && l < top; l++) {
         MgLevel &L = mg->lv[l], &C = mg->lv[l + 1];
-        FX_TRY(smooth(l, mg->n_pre, false));
+        FX_TRY(smooth(l, mg->n_pre, true));
         FX_TRY(ref_restrict_residual(ctx, u_of(l), rhs_of(l), L.rows, L.cols, P[l], B[l], (double *)C.rhs->ptr,
-                                     (double *)C.u->ptr, C.rows, C.cols));
+                                     zero_first(l + 1) ? nullptr : (double *)C.u->ptr, C.rows, C.cols));
     }
-    FX_TRY(smooth(nl - 1, mg->n_pre + mg->n_post + 10, false));
-    for (int l = nl - 2; l >= 0; l--) FX_TRY(smooth(l, mg->n_post, true));
+    if (top < nl)
+        FX_TRY(cheb_tail(ctx, &V[top], &B[top], nl - top, top > 0 || x_zero, mg->n_pre, mg->n_post, n_coarse));
+    else
+        FX_TRY(smooth(nl - 1, n_coarse, true));
+    for (int l = (top < nl ? top : nl - 1) - 1; l >= 0; l--) FX_TRY(smooth(l, mg->n_post, false));
     return own ? fx_copy(ctx, L0.u, x) : FX_OK;
 }
 
