@@ -456,16 +456,135 @@ __global__ void __launch_bounds__(kCdWarps * 32, cd_minb<T>()) k_cd_up(StripGeom
                 cd_smem + (threadIdx.x >> 5) * cd_up_warp_smem<T, TB>());
 }
 
+// ---------------------------------------------------------------- small levels
+//
+// A level with fewer strip chunks than the GPU has warps is pure latency: a march takes seven or
+// more steps of some 1400 cycles (a copy that arrives, two shuffles and three chains of dependent
+// operations each).  Here a block of 16 x 16 own points holds its halo too, one point per thread:
+// one load of everything, then a barrier per stage.  The halo is recomputed (22^2 points down, 20^2
+// up, for 256), which a level that leaves SMs idle gets for nothing.  By strips a level of 33^2 to
+// 129^2 took 7.8 us down and 6.2 us up.
+// Every value is the strip passes' expression.
+
+constexpr int kCdTile = 16;                        // own points per side (even)
+constexpr int kCdTileDown = kCdTile + 6;           // halo 3: x1 -> x2 -> residual -> restriction
+constexpr int kCdTileUp = kCdTile + 4;             // halo 2: f -> x3 -> z
+constexpr int kCdTileDownThreads = (kCdTileDown * kCdTileDown + 31) / 32 * 32;
+constexpr int kCdTileUpThreads = (kCdTileUp * kCdTileUp + 31) / 32 * 32;
+// Levels up to this size go by tiles.  BiCGSTAB on 1025^2 (20 cycles) with the line at 129^2, 257^2,
+// 513^2 and 1025^2: 2967, 2836, 2759 and 3010 us; by strips alone 3490.
+constexpr long long kCdTilePoints = 300000;
+
+template <typename T, typename TB, typename TZ>
+__global__ void __launch_bounds__(kCdTileDownThreads) k_cd_down_tile(CdLevelArgs<T, TB, TZ> L, const int *skip) {
+    grid_dep_enter();
+    if (skip && *(volatile const int *)skip) return;
+    constexpr int W = kCdTileDown;
+    __shared__ T s0[kCdTileDownThreads], s1[kCdTileDownThreads];
+    const int t = threadIdx.x, ty = t / W, tx = t - ty * W;
+    const int r = (int)blockIdx.y * kCdTile - 3 + ty, c = (int)blockIdx.x * kCdTile - 3 + tx;
+    const int rows = L.rows, cols = L.cols;
+    const long long o = (long long)r * cols + c, nf = (long long)rows * cols;
+    const bool in = t < W * W && r >= 1 && r <= rows - 2 && c >= 1 && c <= cols - 2 && FX_IN(o, nf);
+    auto within = [&](int h) { return tx >= h && ty >= h && tx < W - h && ty < W - h; };
+    T b = (T)0, vx = (T)0, vy = (T)0, id = (T)0, x1 = (T)0;
+    if (in) {
+        b = (T)L.b[o];
+        vx = L.vx[o];
+        vy = L.vy[o];
+        id = L.A.inv_diag(vx, vy);
+        x1 = fx_fma(L.omega, b * id, (T)0);
+    }
+    s0[t] = x1;
+    __syncthreads();
+    T x2 = (T)0;
+    if (in && within(1)) {
+        x2 = fx_fma(L.omega, (b - L.A.apply(x1, s0[t - W], s0[t + W], s0[t - 1], s0[t + 1], vx, vy)) * id, x1);
+        if (within(3)) L.x2[o] = x2;
+    }
+    s1[t] = x2;
+    __syncthreads();
+    s0[t] = in && within(2) ? b - L.A.apply(x2, s1[t - W], s1[t + W], s1[t - 1], s1[t + 1], vx, vy) : (T)0;
+    __syncthreads();
+    constexpr int H = kCdTile / 2;
+    if (t < H * H) {
+        const int cy = t / H, cx = t - cy * H;
+        const int fr = (int)blockIdx.y * kCdTile + 2 * cy, fc = (int)blockIdx.x * kCdTile + 2 * cx;
+        const long long oc = (long long)(fr >> 1) * L.ccols + (fc >> 1);
+        if (fr >= 2 && fr <= rows - 3 && fc >= 2 && fc <= cols - 3 && FX_IN(oc, (long long)((rows - 1) / 2 + 1) * L.ccols)) {
+            const T *const q = s0 + (3 + 2 * cy) * W + 3 + 2 * cx;
+            const T e = (q[-W] + q[W]) + (q[-1] + q[1]);
+            const T d = (q[-W - 1] + q[-W + 1]) + (q[W - 1] + q[W + 1]);
+            L.crhs[oc] = ((T)4 * q[0] + ((T)2 * e + d)) * (T)0.0625;
+        }
+    }
+}
+
+template <typename T, typename TB, typename TZ>
+__global__ void __launch_bounds__(kCdTileUpThreads) k_cd_up_tile(CdLevelArgs<T, TB, TZ> L, int zero_ring, const int *skip) {
+    grid_dep_enter();
+    if (skip && *(volatile const int *)skip) return;
+    constexpr int W = kCdTileUp;
+    __shared__ T s0[kCdTileUpThreads], s1[kCdTileUpThreads];
+    const int t = threadIdx.x, ty = t / W, tx = t - ty * W;
+    const int r = (int)blockIdx.y * kCdTile - 2 + ty, c = (int)blockIdx.x * kCdTile - 2 + tx;
+    const int rows = L.rows, cols = L.cols, ccols = L.ccols;
+    const long long o = (long long)r * cols + c, nf = (long long)rows * cols;
+    const bool grid = t < W * W && r >= 0 && r < rows && c >= 0 && c < cols && FX_IN(o, nf);
+    const bool in = grid && r >= 1 && r <= rows - 2 && c >= 1 && c <= cols - 2;
+    auto within = [&](int h) { return tx >= h && ty >= h && tx < W - h && ty < W - h; };
+    T b = (T)0, vx = (T)0, vy = (T)0, id = (T)0, f = (T)0;
+    if (in) {
+        const int crows = (rows - 1) / 2 + 1, m = r >> 1, k = c >> 1;
+        const bool ro = r & 1, co = c & 1;
+        auto at = [&](bool need, int cr, int cc) {
+            const long long oc = (long long)cr * ccols + cc;
+            return need && cr < crows && cc < ccols && FX_IN(oc, (long long)crows * ccols) ? L.e[oc] : (T)0;
+        };
+        const T e00 = at(true, m, k), e01 = at(co, m, k + 1), e10 = at(ro, m + 1, k), e11 = at(ro && co, m + 1, k + 1);
+        const T x2 = L.x2[o];
+        b = (T)L.b[o];
+        vx = L.vx[o];
+        vy = L.vy[o];
+        const T p = ro ? (co ? (T)0.25 * ((e00 + e10) + (e01 + e11)) : (T)0.5 * (e00 + e10))
+                       : (co ? (T)0.5 * (e00 + e01) : e00);
+        f = x2 + p;
+        id = L.A.inv_diag(vx, vy);
+    }
+    s0[t] = f;
+    __syncthreads();
+    T x3 = (T)0;
+    if (in && within(1))
+        x3 = fx_fma(L.omega, (b - L.A.apply(f, s0[t - W], s0[t + W], s0[t - 1], s0[t + 1], vx, vy)) * id, f);
+    s1[t] = x3;
+    __syncthreads();
+    if (!within(2) || !grid) return;
+    if (in)
+        L.z[o] = (TZ)fx_fma(L.omega, (b - L.A.apply(x3, s1[t - W], s1[t + W], s1[t - 1], s1[t + 1], vx, vy)) * id, x3);
+    else if (zero_ring)
+        L.z[o] = (TZ)0;
+}
+
+inline dim3 cd_tiles(int rows, int cols) {
+    return dim3((unsigned)((cols + kCdTile - 1) / kCdTile), (unsigned)((rows + kCdTile - 1) / kCdTile));
+}
+
 template <typename T, typename TB, typename TZ>
 int launch_cd_down(fx_ctx *ctx, const CdLevelArgs<T, TB, TZ> &L, const int *skip) {
     static std::atomic<int> occ{0};
     constexpr size_t smem = kCdWarps * cd_down_warp_smem<T, TB>();
     static_assert(smem <= 48 * 1024, "no opt-in needed");
+    const double pts = (double)L.rows * (double)L.cols;
+    if ((long long)L.rows * L.cols <= kCdTilePoints) {
+        timing_pre(ctx, "cdmg_down");
+        launch_pdl(ctx, k_cd_down_tile<T, TB, TZ>, cd_tiles(L.rows, L.cols), dim3(kCdTileDownThreads), 0, L, skip);
+        timing_post(ctx, pts, pts * (sizeof(TB) + 3.25 * sizeof(T)));
+        return check_launch(ctx, "cdmg_down");
+    }
     const long cap = (long)band_capacity(ctx, k_cd_down<T, TB, TZ>, occ, kCdWarps * 32, smem) * kCdWarps;
     const StripGeom G = strip_geom(L.rows, L.cols, kCdOwnDown, cap);
     timing_pre(ctx, "cdmg_down");
     launch_pdl(ctx, k_cd_down<T, TB, TZ>, (G.nitems + kCdWarps - 1) / kCdWarps, kCdWarps * 32, smem, G, L, skip);
-    const double pts = (double)L.rows * (double)L.cols;
     timing_post(ctx, pts, pts * (sizeof(TB) + 3.25 * sizeof(T)));
     return check_launch(ctx, "cdmg_down");
 }
@@ -474,13 +593,20 @@ template <typename T, typename TB, typename TZ>
 int launch_cd_up(fx_ctx *ctx, const CdLevelArgs<T, TB, TZ> &L, bool zero_ring, const int *skip) {
     static std::atomic<int> occ{0};
     constexpr size_t smem = kCdWarps * cd_up_warp_smem<T, TB>();
+    const double pts = (double)L.rows * (double)L.cols;
+    if ((long long)L.rows * L.cols <= kCdTilePoints) {
+        timing_pre(ctx, "cdmg_up");
+        launch_pdl(ctx, k_cd_up_tile<T, TB, TZ>, cd_tiles(L.rows, L.cols), dim3(kCdTileUpThreads), 0, L, zero_ring ? 1 : 0,
+                   skip);
+        timing_post(ctx, pts, pts * (sizeof(TB) + 3.25 * sizeof(T) + sizeof(TZ)));
+        return check_launch(ctx, "cdmg_up");
+    }
     if (smem > 48 * 1024) FX_TRY(strip_smem_optin(k_cd_up<T, TB, TZ>, smem));
     const long cap = (long)band_capacity(ctx, k_cd_up<T, TB, TZ>, occ, kCdWarps * 32, smem) * kCdWarps;
     const StripGeom G = strip_geom(L.rows, L.cols, kCdOwnUp, cap);
     timing_pre(ctx, "cdmg_up");
     launch_pdl(ctx, k_cd_up<T, TB, TZ>, (G.nitems + kCdWarps - 1) / kCdWarps, kCdWarps * 32, smem, G, L, zero_ring ? 1 : 0,
                skip);
-    const double pts = (double)L.rows * (double)L.cols;
     timing_post(ctx, pts, pts * (sizeof(TB) + 3.25 * sizeof(T) + sizeof(TZ)));
     return check_launch(ctx, "cdmg_up");
 }
