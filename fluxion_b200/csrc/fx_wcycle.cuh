@@ -630,21 +630,132 @@ int strip_smem_optin(K kernel, size_t smem) {
     return FX_OK;
 }
 
+// ---------------------------------------------------------------- small levels
+//
+// A level with fewer strip chunks than the GPU has warps is pure latency: a march of seven or more
+// dependent steps by one warp.  Here a block of 16 x 16 own points holds its halo too, one point per
+// thread: one load of everything, then a barrier per stage.  The halo is recomputed (22^2 points
+// down, 20^2 up, for 256), which a level that leaves SMs idle gets for nothing.
+// Every value is the strip passes' expression.
+
+constexpr int kLvTile = 16;             // own points per side (even)
+constexpr int kTileDown = kLvTile + 6;  // halo 3: x1 -> x2 -> residual -> restriction
+constexpr int kTileUp = kLvTile + 4;    // halo 2: f -> x3 -> z
+constexpr int kTileDownThreads = (kTileDown * kTileDown + 31) / 32 * 32;
+constexpr int kTileUpThreads = (kTileUp * kTileUp + 31) / 32 * 32;
+// Levels up to this size go by tiles.  MG-PCG on 1025 x 1281 with the FP32 cycle, by strips alone and
+// with the line under 257 x 321, over it and over 1025 x 1281: 980, 957, 937 and 1154 us; on 4097^2 in
+// FP64 with the line under 513^2 and over it: 4150 and 4163 us.
+constexpr size_t kTilePoints = 150000;
+
+template <typename T, typename TB>
+__global__ void __launch_bounds__(kTileDownThreads) k_wdown_tile(int rows, int cols, const TB *__restrict__ bg,
+                                                                 T *__restrict__ x2g, T *__restrict__ coarse, int ccols,
+                                                                 VOp<T> op, const int *skip) {
+    grid_dep_enter();
+    if (skip && *(volatile const int *)skip) return;
+    constexpr int W = kTileDown;
+    __shared__ T s0[kTileDownThreads], s1[kTileDownThreads];
+    const int t = threadIdx.x, ty = t / W, tx = t - ty * W;
+    const int r = (int)blockIdx.y * kLvTile - 3 + ty, c = (int)blockIdx.x * kLvTile - 3 + tx;
+    const long long o = (long long)r * cols + c, nf = (long long)rows * cols;
+    (void)nf;
+    const bool in = t < W * W && r >= 1 && r <= rows - 2 && c >= 1 && c <= cols - 2 && FX_IN(o, nf);
+    auto within = [&](int h) { return tx >= h && ty >= h && tx < W - h && ty < W - h; };
+    const T b = in ? (T)bg[o] : (T)0;
+    const T x1 = in ? fx_fma(op.wd, b, (T)0) : (T)0;
+    s0[t] = x1;
+    __syncthreads();
+    T x2 = (T)0;
+    if (in && within(1)) {
+        x2 = fx_fma(op.wd, b - op5v(op.a, x1, s0[t - W], s0[t + W], s0[t - 1], s0[t + 1]), x1);
+        if (within(3)) x2g[o] = x2;
+    }
+    s1[t] = x2;
+    __syncthreads();
+    s0[t] = in && within(2) ? b - op5v(op.a, x2, s1[t - W], s1[t + W], s1[t - 1], s1[t + 1]) : (T)0;
+    __syncthreads();
+    constexpr int H = kLvTile / 2;
+    if (t < H * H) {
+        const int cy = t / H, cx = t - cy * H;
+        const int fr = (int)blockIdx.y * kLvTile + 2 * cy, fc = (int)blockIdx.x * kLvTile + 2 * cx;
+        const long long oc = (long long)(fr >> 1) * ccols + (fc >> 1);
+        if (fr >= 2 && fr <= rows - 3 && fc >= 2 && fc <= cols - 3 && FX_IN(oc, (long long)((rows - 1) / 2 + 1) * ccols)) {
+            const T *const q = s0 + (3 + 2 * cy) * W + 3 + 2 * cx;
+            const T e = (q[-W] + q[W]) + (q[-1] + q[1]);
+            const T d = (q[-W - 1] + q[-W + 1]) + (q[W - 1] + q[W + 1]);
+            coarse[oc] = ((T)4 * q[0] + ((T)2 * e + d)) * (T)0.0625;
+        }
+    }
+}
+
+template <typename T, typename TB, typename TZ>
+__global__ void __launch_bounds__(kTileUpThreads) k_wup_tile(int rows, int cols, const T *__restrict__ x2g,
+                                                             const T *__restrict__ eg, int ccols,
+                                                             const TB *__restrict__ bg, TZ *__restrict__ z, VOp<T> op,
+                                                             const int *skip) {
+    grid_dep_enter();
+    if (skip && *(volatile const int *)skip) return;
+    constexpr int W = kTileUp;
+    __shared__ T s0[kTileUpThreads], s1[kTileUpThreads];
+    const int t = threadIdx.x, ty = t / W, tx = t - ty * W;
+    const int r = (int)blockIdx.y * kLvTile - 2 + ty, c = (int)blockIdx.x * kLvTile - 2 + tx;
+    const int crows = (rows - 1) / 2 + 1;
+    const long long o = (long long)r * cols + c, nf = (long long)rows * cols, nc = (long long)crows * ccols;
+    (void)nf;
+    (void)nc;
+    const bool in = t < W * W && r >= 1 && r <= rows - 2 && c >= 1 && c <= cols - 2 && FX_IN(o, nf);
+    auto within = [&](int h) { return tx >= h && ty >= h && tx < W - h && ty < W - h; };
+    T b = (T)0, f = (T)0;
+    if (in) {
+        const int m = r >> 1, k = c >> 1;
+        const bool ro = r & 1, co = c & 1;
+        auto at = [&](bool need, int cr, int cc) {
+            const long long oc = (long long)cr * ccols + cc;
+            return need && cr < crows && cc < ccols && FX_IN(oc, nc) ? eg[oc] : (T)0;
+        };
+        const T e00 = at(true, m, k), e01 = at(co, m, k + 1), e10 = at(ro, m + 1, k), e11 = at(ro && co, m + 1, k + 1);
+        const T x2 = x2g[o];
+        b = (T)bg[o];
+        f = x2 + (ro ? (co ? (T)0.25 * ((e00 + e10) + (e01 + e11)) : (T)0.5 * (e00 + e10))
+                     : (co ? (T)0.5 * (e00 + e01) : e00));
+    }
+    s0[t] = f;
+    __syncthreads();
+    T x3 = (T)0;
+    if (in && within(1)) x3 = fx_fma(op.wd, b - op5v(op.a, f, s0[t - W], s0[t + W], s0[t - 1], s0[t + 1]), f);
+    s1[t] = x3;
+    __syncthreads();
+    if (in && within(2)) z[o] = (TZ)fx_fma(op.wd, b - op5v(op.a, x3, s1[t - W], s1[t + W], s1[t - 1], s1[t + 1]), x3);
+}
+
+inline dim3 level_tiles(size_t rows, size_t cols) {
+    return dim3((unsigned)((cols + kLvTile - 1) / kLvTile), (unsigned)((rows + kLvTile - 1) / kLvTile));
+}
+
 template <typename T, typename TB>
 int launch_wdown(fx_ctx *ctx, size_t rows, size_t cols, const TB *b, T *x2, T *coarse, size_t ccols,
                  const VOp<T> &op, const int *skip, int chunk_pct = 100) {
     static std::atomic<int> occ{0};
     constexpr int W = strip_warps<T>();
     constexpr size_t smem = wdown_smem<T, TB>();
+    // reads b, writes the smoothed x2 and the restricted coarse rhs
+    const double pts = (double)rows * (double)cols, cpts = (double)((rows - 1) / 2 + 1) * (double)ccols;
+    const double bytes = pts * (sizeof(TB) + sizeof(T)) + cpts * sizeof(T);
+    if (rows * cols <= kTilePoints) {
+        timing_pre(ctx, "mg_down");
+        launch_pdl(ctx, k_wdown_tile<T, TB>, level_tiles(rows, cols), dim3(kTileDownThreads), 0, (int)rows, (int)cols, b, x2,
+                   coarse, (int)ccols, op, skip);
+        timing_post(ctx, pts, bytes);
+        return check_launch(ctx, "mg_down");
+    }
     if (smem > 48 * 1024) FX_TRY(strip_smem_optin(k_wdown<T, TB>, smem));
     const long cap = strip_capacity((long)band_capacity(ctx, k_wdown<T, TB>, occ, W * 32, smem) * W, chunk_pct);
     const StripGeom G = strip_geom(rows, cols, kDownOwn, cap);
     const int blocks = (G.nitems + W - 1) / W;
     timing_pre(ctx, "mg_down");
     launch_pdl(ctx, k_wdown<T, TB>, blocks, W * 32, smem, G, b, x2, coarse, (int)ccols, op, skip);
-    // reads b, writes the smoothed x2 and the restricted coarse rhs
-    const double pts = (double)rows * (double)cols, cpts = (double)((rows - 1) / 2 + 1) * (double)ccols;
-    timing_post(ctx, pts, pts * (sizeof(TB) + sizeof(T)) + cpts * sizeof(T));
+    timing_post(ctx, pts, bytes);
     return check_launch(ctx, "mg_down");
 }
 
@@ -654,6 +765,18 @@ int launch_wup(fx_ctx *ctx, size_t rows, size_t cols, const T *x2, const T *e, s
     static std::atomic<int> occ{0};
     constexpr int W = strip_warps<T>();
     constexpr size_t smem = wup_smem<T, TB>();
+    // reads x2, the coarse correction e and b, writes z
+    const double pts = (double)rows * (double)cols, cpts = (double)((rows - 1) / 2 + 1) * (double)ccols;
+    const double bytes = pts * (sizeof(T) + sizeof(TB) + sizeof(TZ)) + cpts * sizeof(T);
+    if constexpr (!RZ) {
+        if (rows * cols <= kTilePoints) {
+            timing_pre(ctx, "mg_up");
+            launch_pdl(ctx, k_wup_tile<T, TB, TZ>, level_tiles(rows, cols), dim3(kTileUpThreads), 0, (int)rows, (int)cols, x2,
+                       e, (int)ccols, b, z, op, skip);
+            timing_post(ctx, pts, bytes);
+            return check_launch(ctx, "mg_up");
+        }
+    }
     if (smem > 48 * 1024) FX_TRY(strip_smem_optin(k_wup<T, TB, TZ, RZ, Fin>, smem));
     const long cap =
         strip_capacity((long)band_capacity(ctx, k_wup<T, TB, TZ, RZ, Fin>, occ, W * 32, smem) * W, chunk_pct);
@@ -663,9 +786,7 @@ int launch_wup(fx_ctx *ctx, size_t rows, size_t cols, const T *x2, const T *e, s
     timing_pre(ctx, "mg_up");
     launch_pdl(ctx, k_wup<T, TB, TZ, RZ, Fin>, blocks, W * 32, smem, G, x2, e, (int)ccols, b, z, op, fin,
                red_args<1>(ctx), skip);
-    // reads x2, the coarse correction e and b, writes z
-    const double pts = (double)rows * (double)cols, cpts = (double)((rows - 1) / 2 + 1) * (double)ccols;
-    timing_post(ctx, pts, pts * (sizeof(T) + sizeof(TB) + sizeof(TZ)) + cpts * sizeof(T));
+    timing_post(ctx, pts, bytes);
     return check_launch(ctx, "mg_up");
 }
 
