@@ -2795,8 +2795,8 @@ int check_op(const fx_grid &g, const fx_op *op) {
 // multigrid).  Each coarse level rediscretises the operator with h doubled and kappa / vx / vy
 // injected from the coincident fine points.  Smoother: x <- x + omega (b - A x) / diag(A)
 // inside; full weighting down, bilinear up; `coarse_sweeps` sweeps on the coarsest level in
-// one block; every cycle from x = 0.  Unfused (a sweep, residual and transfer pass each): the
-// variable coefficients do not fit the constant-stencil level kernels.
+// one block; every cycle from x = 0.  With a scalar kappa and V(2,2) a level is a down and an up
+// pass (fx_cdcycle.cuh); otherwise a sweep, residual and transfer pass each.
 
 template <typename T>
 __device__ __forceinline__ T cd_diag(const OpA<T, kModeCD> &A, size_t idx) {
