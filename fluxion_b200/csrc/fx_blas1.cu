@@ -275,11 +275,29 @@ int fx_norm_l2(fx_ctx *ctx, const fx_buf *buf, double *out) {
     }
     FX_DISPATCH(buf->dtype, {
         const T *p = (const T *)buf->ptr;
-        FX_TRY(launch_flat<1>(ctx, buf->len,
-                              [=] __device__(size_t i, CSum *acc) {
-                                  csum_add_prod_t<T>(acc[0], p[i], p[i]);
-                              },
-                              StoreFin<1>{ctx->d_result}, nullptr, "norm_l2"));
+        // four FP32 elements a load, as the dot: with one the loads in flight bound it (residual and
+        // norm of 8191 x 6001: 363 us, and 316 so)
+        bool vec = false;
+        if constexpr (sizeof(T) == 4) {
+            if (aligned16(p) && buf->len >= 4096) {
+                vec = true;
+                FX_TRY(launch_vec4<1>(
+                    ctx, buf->len,
+                    [=] __device__(size_t j, CSum *acc) {
+                        const float4 a = reinterpret_cast<const float4 *>(p)[j];
+                        csum_add_prod_t<float>(acc[0], a.x, a.x);
+                        csum_add_prod_t<float>(acc[0], a.y, a.y);
+                        csum_add_prod_t<float>(acc[0], a.z, a.z);
+                        csum_add_prod_t<float>(acc[0], a.w, a.w);
+                    },
+                    [=] __device__(size_t i, CSum *acc) { csum_add_prod_t<float>(acc[0], p[i], p[i]); },
+                    StoreFin<1>{ctx->d_result}, "norm_l2"));
+            }
+        }
+        if (!vec)
+            FX_TRY(launch_flat<1>(ctx, buf->len,
+                                  [=] __device__(size_t i, CSum *acc) { csum_add_prod_t<T>(acc[0], p[i], p[i]); },
+                                  StoreFin<1>{ctx->d_result}, nullptr, "norm_l2"));
     });
     FX_TRY(read_results(ctx, 1, out));
     *out = sqrt(*out);
