@@ -292,9 +292,11 @@ class DiffusionSolver:
         self._use_graph = True
 
     def _fused(self, u: Field, n: int) -> bool:
-        """`n` steps without a source in the library's fused passes, where these hold: zero Dirichlet
-        sides, F64 (fx_diffusion_steps; the same values as the sequence of field operations)."""
-        if n < 1 or not self.boundaries.is_zero_dirichlet() or u.dtype() != DType.F64 or u.grid() != self.grid:
+        """`n` steps without a source in the library's fused passes, where these hold: a five-point
+        stencil, zero Dirichlet sides, F64 (fx_diffusion_steps; the same values as the sequence of
+        field operations)."""
+        if (n < 1 or self.stencil.len() != 5 or not self.boundaries.is_zero_dirichlet() or u.dtype() != DType.F64
+                or u.grid() != self.grid):
             return False
         u._same(self.scratch[0])
         self.device.backend().diffusion_steps(u.storage, self.scratch[0].storage, self.grid, self.stencil, self.alpha,

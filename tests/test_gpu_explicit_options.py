@@ -1,0 +1,47 @@
+"""Options of the explicit stepper around its fused passes: what the passes do not hold runs as the
+sequence of field operations, with the same results as ever."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def dev():
+    from fluxion_b200 import Device
+    return Device.best()
+
+
+def _solver(g, scheme, dev, boundaries=None, stencil=None):
+    from fluxion_b200 import Boundaries
+    from fluxion_b200.steppers import DiffusionSolver, TimeScheme
+    s = DiffusionSolver.build(g, 0.7, None, boundaries or Boundaries.zero_dirichlet(), TimeScheme[scheme], dev)
+    if stencil is not None:
+        s.stencil = stencil
+    return s
+
+
+def _grid_and_data(rows=37, cols=50):
+    from fluxion_b200 import Grid
+    h = 1.0 / (max(rows, cols) - 1)
+    return Grid.new(rows, cols, h, 1.5 * h), np.random.default_rng(rows * cols).uniform(-1, 1, rows * cols)
+
+
+@pytest.mark.parametrize("scheme", ["Euler", "Rk2", "Rk4"])
+@pytest.mark.parametrize("entries", ["nine", "three", "five, another order"])
+def test_other_stencils(dev, scheme, entries):
+    """A solver whose stencil is not the five-point form steps by the field operations; five entries in
+    any order are the five-point form."""
+    from fluxion_b200 import Field, Stencil
+    g, data = _grid_and_data()
+    five = Stencil.laplacian_2d_5pt(g.dx, g.dy)
+    stencil = {"nine": Stencil.laplacian_2d_9pt(g.dx, g.dy), "three": Stencil(five.as_triples()[:3]),
+               "five, another order": Stencil(five.as_triples()[::-1])}[entries]
+    a, b = (_solver(g, scheme, dev, stencil=stencil) for _ in range(2))
+    ua, ub = Field.from_f64(g, data, dev), Field.from_f64(g, data, dev)
+    a.step_n(ua, 3)
+    a.step(ua)
+    for _ in range(4):
+        b._record(ub, None)
+    assert a.steps_done() == 4
+    assert np.array_equal(ua.to_vec_f64(), ub.to_vec_f64())
