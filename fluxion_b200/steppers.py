@@ -242,8 +242,10 @@ class DiffusionSolver:
     classical RK4, each stage the reference's sequence of field operations (in fused passes for zero
     Dirichlet sides and no source, with the same values).  The default dt is
     the reference's stability bound safety * h_min^2 / (4 alpha) (safety 0.4 / 0.8 / 1.4).
-    ``enable_graph()`` is the HipGraph path (solver.rs:182-325) on CUDA graphs: the first
-    ``step_n`` records one step on the backend's stream and later steps replay it."""
+    ``enable_graph()`` is the HipGraph path (solver.rs:182-325) on CUDA graphs: the first ``step_n``
+    fixes the step and its field, and later calls repeat it whatever the solver's attributes are by
+    then.  A step of field operations is recorded on the backend's stream and replayed; one of the
+    fused passes is a launch or two as it is, and its arguments are kept instead."""
 
     def __init__(self, grid: Grid, alpha: float, dt: Optional[float], boundaries: Boundaries,
                  scheme: "TimeScheme", device: Optional[Device] = None):
@@ -291,53 +293,61 @@ class DiffusionSolver:
         """solver.rs:182-186 (enable_hip_graph)."""
         self._use_graph = True
 
-    def _fused(self, u: Field, n: int) -> bool:
-        """`n` steps without a source in the library's fused passes, where these hold: a five-point
-        stencil, zero Dirichlet sides, F64 (fx_diffusion_steps; the same values as the sequence of
-        field operations)."""
-        if (n < 1 or self.stencil.len() != 5 or not self.boundaries.is_zero_dirichlet() or u.dtype() != DType.F64
+    def _passes(self, u: Field) -> Optional[tuple]:
+        """A step of u without a source as the arguments of the library's fused passes, where these
+        hold: a five-point stencil, zero Dirichlet sides, F64 (fx_diffusion_steps; the same values as
+        the sequence of field operations)."""
+        if (self.stencil.len() != 5 or not self.boundaries.is_zero_dirichlet() or u.dtype() != DType.F64
                 or u.grid() != self.grid):
-            return False
+            return None
         u._same(self.scratch[0])
-        self.device.backend().diffusion_steps(u.storage, self.scratch[0].storage, self.grid, self.stencil, self.alpha,
-                                              self._dt, self._scheme.value, n)
-        self._steps_done += n
-        return True
+        return (u.storage, self.scratch[0].storage, self.grid, self.stencil, self.alpha, self._dt, self._scheme.value)
 
     def step(self, u: Field, source: Optional[Field] = None) -> None:
-        if source is None and self._fused(u, 1):
-            return
-        self._record(u, source)
+        passes = self._passes(u) if source is None else None
+        if passes is not None:
+            self.device.backend().diffusion_steps(*passes, 1)
+        else:
+            self._record(u, source)
         self._steps_done += 1
 
     def step_n(self, u: Field, n: int) -> None:
-        """solver.rs:231-257; with the graph enabled, the recorded step is replayed n times
-        (one graph per solver, recorded on the first field passed)."""
+        """solver.rs:231-257; with the graph enabled, the first call's step is repeated n times (one
+        step per solver, on the first field passed)."""
         if n == 0:
             return
-        if not self._use_graph and self._fused(u, n):
-            return
         if self._use_graph:
-            # the fused passes need no recording; the solver stays with the first field all the same
-            if self._graph is None and self._graph_u in (None, u) and self._fused(u, n):
-                self._graph_u = u
-                return
-            if self._graph is None and self._graph_u is None:
-                be = self.device.backend()
-                be.graph_begin()
-                try:
-                    self._record(u, None)
-                finally:
-                    self._graph = be.graph_end()
+            if self._graph is None:
+                # the fused passes have nothing to record: their arguments are the step
+                self._graph = self._passes(u)
+                if self._graph is None:
+                    be = self.device.backend()
+                    be.graph_begin()
+                    try:
+                        self._record(u, None)
+                    finally:
+                        self._graph = be.graph_end()
                 self._graph_u = u
             if u is not self._graph_u:
                 raise ValueError("the recorded step belongs to another field")
+            if isinstance(self._graph, tuple):
+                self._repeat(self._graph, n)
+                return
             for _ in range(n):
                 self._graph.launch()
                 self._steps_done += 1
             return
+        passes = self._passes(u)
+        if passes is not None:
+            self._repeat(passes, n)
+            return
         for _ in range(n):
             self.step(u, None)
+
+    def _repeat(self, passes: tuple, n: int) -> None:
+        if n > 0:
+            self.device.backend().diffusion_steps(*passes, n)
+            self._steps_done += n
 
     def step_n_with_source(self, u: Field, n: int, source: Field) -> None:
         for _ in range(n):

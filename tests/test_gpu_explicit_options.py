@@ -45,3 +45,35 @@ def test_other_stencils(dev, scheme, entries):
         b._record(ub, None)
     assert a.steps_done() == 4
     assert np.array_equal(ua.to_vec_f64(), ub.to_vec_f64())
+
+
+def _boundaries(kind):
+    from fluxion_b200 import BoundaryCondition, Boundaries
+    return {"zero Dirichlet": Boundaries.zero_dirichlet(),
+            "Dirichlet": Boundaries(*[BoundaryCondition.Dirichlet(v) for v in (0.3, -0.2, 0.0, 0.7)]),
+            "mixed": Boundaries(BoundaryCondition.Neumann(0.5), BoundaryCondition.Robin(1.0, 2.0, 0.3),
+                                BoundaryCondition.Dirichlet(0.7), BoundaryCondition.Neumann(-0.2))}[kind]
+
+
+@pytest.mark.parametrize("scheme", ["Euler", "Rk2", "Rk4"])
+@pytest.mark.parametrize("kind", ["zero Dirichlet", "Dirichlet", "mixed"])
+def test_graph_solver_repeats_its_first_step(dev, scheme, kind):
+    """With the graph enabled the first step_n fixes the step: later calls repeat it on the same field,
+    whatever the solver's attributes are by then, and the result is that of the field operations."""
+    from fluxion_b200 import Field, Stencil
+    g, data = _grid_and_data()
+    a, b = (_solver(g, scheme, dev, _boundaries(kind)) for _ in range(2))
+    ua, ub = Field.from_f64(g, data, dev), Field.from_f64(g, data, dev)
+    a.enable_graph()
+    a.step_n(ua, 10)
+    with pytest.raises(ValueError):
+        a.step_n(Field.from_f64(g, data, dev), 1)
+    a.boundaries = _boundaries("Dirichlet" if kind == "mixed" else "mixed")
+    a.step_n(ua, 7)
+    a.boundaries = _boundaries("zero Dirichlet")
+    a.alpha, a.stencil = 0.3, Stencil.laplacian_2d_9pt(g.dx, g.dy)
+    a.step_n(ua, 8)
+    for _ in range(25):
+        b._record(ub, None)
+    assert a.steps_done() == 25
+    assert np.array_equal(ua.to_vec_f64(), ub.to_vec_f64())
