@@ -316,6 +316,7 @@ class DiffusionSolver:
         step per solver, on the first field passed)."""
         if n == 0:
             return
+        n = len(range(n))  # an integer; a negative one counts as none
         if self._use_graph:
             if self._graph is None:
                 # the fused passes have nothing to record: their arguments are the step
@@ -337,7 +338,7 @@ class DiffusionSolver:
                 self._graph.launch()
                 self._steps_done += 1
             return
-        passes = self._passes(u)
+        passes = self._passes(u) if n else None
         if passes is not None:
             self._repeat(passes, n)
             return
@@ -345,9 +346,8 @@ class DiffusionSolver:
             self.step(u, None)
 
     def _repeat(self, passes: tuple, n: int) -> None:
-        if n > 0:
-            self.device.backend().diffusion_steps(*passes, n)
-            self._steps_done += n
+        self.device.backend().diffusion_steps(*passes, n)
+        self._steps_done += n
 
     def step_n_with_source(self, u: Field, n: int, source: Field) -> None:
         for _ in range(n):

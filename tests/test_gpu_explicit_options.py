@@ -77,3 +77,21 @@ def test_graph_solver_repeats_its_first_step(dev, scheme, kind):
         b._record(ub, None)
     assert a.steps_done() == 25
     assert np.array_equal(ua.to_vec_f64(), ub.to_vec_f64())
+
+
+@pytest.mark.parametrize("graph", [False, True])
+@pytest.mark.parametrize("kind", ["zero Dirichlet", "mixed"])
+def test_step_counts(dev, graph, kind):
+    """A step count is an integer: another number is refused and a negative one makes no step."""
+    from fluxion_b200 import Field
+    g, data = _grid_and_data()
+    s, u = _solver(g, "Euler", dev, _boundaries(kind)), Field.from_f64(g, data, dev)
+    if graph:
+        s.enable_graph()
+    with pytest.raises(TypeError):
+        s.step_n(u, 2.5)
+    s.step_n(u, -3)
+    s.step_n(u, 0)
+    assert s.steps_done() == 0 and np.array_equal(u.to_vec_f64(), data)
+    s.step_n(u, np.int64(2))
+    assert s.steps_done() == 2
