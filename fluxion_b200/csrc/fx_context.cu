@@ -99,6 +99,20 @@ bool capturing(cudaStream_t s) {
     return cs != cudaStreamCaptureStatusNone;
 }
 
+int zero_scratch(fx_ctx *ctx, void *p, size_t bytes) {
+    if (!capturing(ctx->stream)) {
+        FX_CUDA(cudaMemsetAsync(p, 0, bytes, ctx->stream));
+        return FX_OK;
+    }
+    cudaStream_t s;  // a memset on a captured stream would only run with the graph
+    FX_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+    cudaError_t e = cudaMemsetAsync(p, 0, bytes, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    cudaStreamDestroy(s);
+    FX_CUDA(e);
+    return FX_OK;
+}
+
 void timing_pre(fx_ctx *ctx, const char *what) {
     if (!ctx->timing || ctx->timing_name != what) return;
     if (ctx->pool_next + 2 > ctx->event_pool.size()) {
@@ -369,7 +383,7 @@ int fx_ctx_create(int device, fx_ctx **out) {
         cudaMalloc(&c->d_result, sizeof(double) * 8) != cudaSuccess ||
         cudaHostAlloc(&c->h_result, sizeof(double) * 8, cudaHostAllocMapped) != cudaSuccess ||
         cudaHostGetDevicePointer((void **)&c->h_result_dev, c->h_result, 0) != cudaSuccess ||
-        cudaMemset(c->d_counter, 0, sizeof(unsigned) * 4) != cudaSuccess) {
+        cudaMemsetAsync(c->d_counter, 0, sizeof(unsigned) * 4, c->own_stream) != cudaSuccess) {
         std::string m = cudaGetErrorString(cudaGetLastError());
         fx_ctx_destroy(c);
         return fail(FX_ERR_BACKEND, "context allocation failed: " + m);

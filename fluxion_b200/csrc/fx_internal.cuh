@@ -170,6 +170,9 @@ struct NvtxRange {
 };
 #define FX_RANGE(name) ::fx::NvtxRange fx_nvtx_range_(name)
 bool capturing(cudaStream_t s);  // the stream is being captured into a graph
+// Zero a fresh device allocation before the context's next kernels.  Its stream does not wait for the
+// default stream, so a plain memset there could land after them.
+int zero_scratch(fx_ctx *ctx, void *p, size_t bytes);
 
 // Programmatic dependent launch.  Kernels of the solve path are launched with programmatic
 // stream serialisation, so the next kernel's launch and block scheduling overlap the end of

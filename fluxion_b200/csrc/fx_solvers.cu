@@ -2069,9 +2069,9 @@ int mgs_two_pass(fx_gmres *s, size_t n, double *w, const std::vector<double *> &
 int mgs_alloc(fx_gmres *s) {
     const size_t words = (size_t)kMgsMax * kMgsMax + (size_t)s->ctx->num_sms * 8 * 4 * kMgsGroup;
     FX_CUDA(cudaMalloc(&s->d_mgs, words * sizeof(double)));
-    FX_CUDA(cudaMemset(s->d_mgs, 0, words * sizeof(double)));
+    FX_TRY(zero_scratch(s->ctx, s->d_mgs, words * sizeof(double)));
     FX_CUDA(cudaMalloc(&s->d_mgs_ticket, sizeof(unsigned)));
-    FX_CUDA(cudaMemset(s->d_mgs_ticket, 0, sizeof(unsigned)));
+    FX_TRY(zero_scratch(s->ctx, s->d_mgs_ticket, sizeof(unsigned)));
     return FX_OK;
 }
 
@@ -4184,7 +4184,7 @@ int fx_fgmres_set_orthogonalization(fx_fgmres *s, int method) {
         if (cudaMalloc(&s->d_cgs, 2 * (s->restart + 2) * sizeof(double)) != cudaSuccess ||
             cudaMalloc(&s->d_part, blocks * kCgsMax * sizeof(double)) != cudaSuccess ||
             cudaMalloc(&s->d_ticket, sizeof(unsigned)) != cudaSuccess ||
-            cudaMemset(s->d_ticket, 0, sizeof(unsigned)) != cudaSuccess) {
+            zero_scratch(s->ctx, s->d_ticket, sizeof(unsigned)) != FX_OK) {
             (void)cudaGetLastError();
             return fail(FX_ERR_BACKEND, "fgmres CGS2 scratch allocation failed");
         }
@@ -4420,13 +4420,13 @@ int fx_cdmg_set_learned(fx_cdmg *mg, const fx_lsm *lsm, size_t min_points, size_
         FX_CUDA(cudaMalloc(&mg->d_lsm_scale, 2 * sizeof(double)));
         FX_CUDA(cudaMalloc(&mg->d_plain_skip, sizeof(int)));
         FX_CUDA(cudaMalloc(&mg->d_lsm_counts, 2 * sizeof(unsigned long long)));
-        FX_CUDA(cudaMemset(mg->d_lsm_counts, 0, 2 * sizeof(unsigned long long)));
+        FX_TRY(zero_scratch(mg->ctx, mg->d_lsm_counts, 2 * sizeof(unsigned long long)));
     }
     mg->lsm = lsm;
     mg->lsm_min_points = min_points;
     mg->lsm_max_points = max_points;
     mg->lsm_ratio = fallback_ratio;
-    if (mg->d_lsm_state) FX_CUDA(cudaMemset(mg->d_lsm_state, 0, 3 * sizeof(int)));
+    if (mg->d_lsm_state) FX_TRY(zero_scratch(mg->ctx, mg->d_lsm_state, 3 * sizeof(int)));
     return FX_OK;
 }
 
@@ -4435,7 +4435,7 @@ int fx_cdmg_set_learned_patience(fx_cdmg *mg, size_t patience) {
     if (patience > (size_t)1 << 30) return fail(FX_ERR_INVALID_ARGUMENT, "patience out of range");
     FX_CUDA(cudaStreamSynchronize(mg->ctx->stream));
     if (!mg->d_lsm_state) FX_CUDA(cudaMalloc(&mg->d_lsm_state, 3 * sizeof(int)));
-    FX_CUDA(cudaMemset(mg->d_lsm_state, 0, 3 * sizeof(int)));
+    FX_TRY(zero_scratch(mg->ctx, mg->d_lsm_state, 3 * sizeof(int)));
     if ((int)patience != mg->lsm_patience) mg->drop_replays();  // the gate joins or leaves the sequence
     mg->lsm_patience = (int)patience;
     return FX_OK;
