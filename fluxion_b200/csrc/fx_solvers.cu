@@ -1847,16 +1847,18 @@ struct FlatGmMgs {  // w -= h_j v_j; reduction w.v_{j+1} (or w.w after the last)
 // coefficients up to rounding, 16 B/point per vector:
 //   dots:   s_j = v_j . w and row k of L, v_j . v_k, in one pass; the last block solves for h;
 //   update: w -= sum_j h_j v_j, element by element in MGS's order, and ||w||^2.
-// s_j and ||w||^2 are sums of exact products, as MGS's dots; the entries of L (of rounding size, and
-// multiplying h) are per-thread fma partials folded compensated.
+// s_j, ||w||^2 and the entries of L are compensated sums of exact products, as MGS's dots, and the
+// triangular solve carries two words, so h is rounded once and its error is the rounding of w in
+// either form.  Iterates against an 80-bit GMRES, 400 random systems of 64 to 250 points a side, 9 to
+// 60 iterations: 6.67e-16 relative in the mean here, 6.64e-16 with a pass per vector; attained
+// residuals on operators of condition 1e7 to 1e8 (200 of them): 0.99 of the others' in the mean.
 //
-// Dots: a block takes a group of up to 8 basis vectors (its threads hold 8 compensated sums) over a
+// Dots: a block takes a group of up to 8 basis vectors (its threads hold 8 pairs of sums) over a
 // share of the elements, so w and v_k are read once per group, mostly from L2; groups are of equal
-// size, and their registers are capped for two blocks per SM (three for up to 5 vectors): 1.44 ms an
-// iteration of FGMRES(30) with the fused cycle at 4097 x 4097 without the cap, 1.35 with it.  Against
-// a pass per vector: 1.84 ms an iteration there, 42 against 92 us for GMRES(30) at 129 x 131 (two
-// launches a step instead of k + 1), 249 against 446 at 2049 x 2049.  Two sums per 8 bytes read are
-// half of the FP64 rate at the HBM rate; both passes run within 10 % of it.
+// size, and their registers are capped for two blocks per SM (three for up to 4 vectors; 5 spill at
+// three).  Against a pass per vector: 42 us an iteration of GMRES(30) at 129 x 131, from 91 (two
+// launches a step instead of k + 1), 126 from 203 at 1021 x 1531, 266 from 441 at 2049 x 2049.  The
+// dots are 14 FP64 operations for 8 bytes from HBM, 0.6 of the FP64 rate at the HBM rate.
 constexpr int kMgsMax = 32;   // basis vectors (above, and for one vector, a pass per vector)
 constexpr int kMgsGroup = 8;  // vectors per block
 
@@ -1871,8 +1873,19 @@ struct MgsArgs {
     double *h;    // [kb + 1]: the coefficients, then ||w||^2
 };
 
+// acc += a b for the dot of two unit vectors.  No partial of it exceeds 1 (Cauchy-Schwarz), so with a
+// bias of 3 the running sum stays in [2, 4]: it moves by a multiple of its last place, the difference
+// of two of its values is exact, and so is what a b has beyond that up to a rounding of 2^-105.  Four
+// operations, against csum_add_prod's ten, for a sum whose size is not known beforehand.
+constexpr double kUnitBias = 3.0;
+__device__ __forceinline__ void unit_dot_add(CSum &acc, double a, double b) {
+    const double s = fma(a, b, acc.s);
+    acc.c += fma(a, b, acc.s - s);
+    acc.s = s;
+}
+
 template <int GS>
-__global__ void __launch_bounds__(kBlock, GS >= 6 ? 2 : 3) k_mgs_dots(size_t n, MgsArgs a) {
+__global__ void __launch_bounds__(kBlock, GS >= 5 ? 2 : 3) k_mgs_dots(size_t n, MgsArgs a) {
     grid_dep_enter();
     const int grp = blockIdx.x % a.ng, lb = blockIdx.x / a.ng;
     const int nbg = (gridDim.x - grp + a.ng - 1) / a.ng;  // blocks of this group
@@ -1883,7 +1896,7 @@ __global__ void __launch_bounds__(kBlock, GS >= 6 ? 2 : 3) k_mgs_dots(size_t n, 
     const double *vk = a.v[a.kb - 1];
     CSum acc[2 * GS];
 #pragma unroll
-    for (int q = 0; q < 2 * GS; q++) acc[q] = CSum{0.0, 0.0};
+    for (int q = 0; q < 2 * GS; q++) acc[q] = CSum{q < GS ? 0.0 : kUnitBias, 0.0};
     const size_t stride = (size_t)nbg * kBlock;
     size_t i = (size_t)lb * kBlock + threadIdx.x;
     for (; i + stride < n; i += 2 * stride) {  // two elements' loads in flight
@@ -1900,7 +1913,7 @@ __global__ void __launch_bounds__(kBlock, GS >= 6 ? 2 : 3) k_mgs_dots(size_t n, 
 #pragma unroll
             for (int q = 0; q < GS; q++) {
                 csum_add_prod(acc[q], e[u][q], x[u]);
-                csum_fma(acc[GS + q], e[u][q], y[u]);
+                unit_dot_add(acc[GS + q], e[u][q], y[u]);
             }
     }
     if (i < n) {
@@ -1909,9 +1922,11 @@ __global__ void __launch_bounds__(kBlock, GS >= 6 ? 2 : 3) k_mgs_dots(size_t n, 
         for (int q = 0; q < GS; q++) {
             const double e = v[q][i];
             csum_add_prod(acc[q], e, x);
-            csum_fma(acc[GS + q], e, y);
+            unit_dot_add(acc[GS + q], e, y);
         }
     }
+#pragma unroll
+    for (int q = GS; q < 2 * GS; q++) acc[q].s -= kUnitBias;  // exact
     block_reduce<2 * GS>(acc);
     __shared__ bool is_last;
     if (threadIdx.x == 0) {
@@ -1930,7 +1945,7 @@ __global__ void __launch_bounds__(kBlock, GS >= 6 ? 2 : 3) k_mgs_dots(size_t n, 
     if (!is_last) return;
     __threadfence();
     // the last block: fold each vector's partials in block order (a warp per vector), then solve
-    __shared__ double s[kMgsMax], Lm[kMgsMax][kMgsMax + 1];
+    __shared__ double s[kMgsMax], sc[kMgsMax], Lm[kMgsMax][kMgsMax + 1];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, kb = a.kb;
     for (int t = threadIdx.x; t < (kb - 1) * kMgsMax; t += kBlock) Lm[t / kMgsMax][t % kMgsMax] = a.L[t];
     for (int j = wid; j < kb; j += kBlock / 32) {
@@ -1953,7 +1968,7 @@ __global__ void __launch_bounds__(kBlock, GS >= 6 ? 2 : 3) k_mgs_dots(size_t n, 
             l = csum_merge(l, o);
         }
         if (lane == 0) {
-            s[j] = csum_value(d);
+            two_sum(d.s, d.c, s[j], sc[j]);
             if (j < kb - 1) {
                 const double lv = csum_value(l);
                 Lm[kb - 1][j] = lv;
@@ -1962,13 +1977,19 @@ __global__ void __launch_bounds__(kBlock, GS >= 6 ? 2 : 3) k_mgs_dots(size_t n, 
         }
     }
     __syncthreads();
-    if (wid == 0) {  // h_j = s_j - sum_{i < j} L_ji h_i, a column at a time
-        double r = lane < kb ? s[lane] : 0.0;
+    if (wid == 0) {  // h_j = s_j - sum_{i < j} L_ji h_i, a column at a time; h_j rounded once, when it is done
+        double r = lane < kb ? s[lane] : 0.0, rc = lane < kb ? sc[lane] : 0.0;
         for (int i = 0; i + 1 < kb; i++) {
-            const double hi = __shfl_sync(0xffffffffu, r, i);
-            if (lane > i && lane < kb) r = fma(-Lm[lane][i], hi, r);
+            const double hi = __shfl_sync(0xffffffffu, r + rc, i);
+            if (lane > i && lane < kb) {
+                const double p = -Lm[lane][i] * hi;
+                double t, e;
+                two_sum(r, p, t, e);
+                r = t;
+                rc += e + fma(-Lm[lane][i], hi, -p);
+            }
         }
-        if (lane < kb) a.h[lane] = r;
+        if (lane < kb) a.h[lane] = r + rc;
     }
     if (threadIdx.x == 0) *a.ticket = 0u;
 }
