@@ -3295,8 +3295,8 @@ struct fx_cdmg {
         bool writes_all() const override { return mg->fused(0, false) && !mg->lsm; }
     } view;
     // One application is a fixed sequence of launches for given (z, r, halt flag, stream).  With
-    // replay on (fx_cdmg_set_replay), it is recorded into a CUDA graph the first time and
-    // replayed after that: one launch instead of 20-50.  Off by default: recording and
+    // replay on (fx_cdmg_set_replay), it is launched and recorded into a CUDA graph the first time
+    // and replayed after that: one launch instead of 7 or more.  Off by default: recording and
     // instantiating costs more than a short-lived hierarchy's replays save (the batched
     // workload, one new hierarchy per problem, same box: -5 % on one lane, -4 to -9 % on 8).
     struct Replay {
@@ -3338,11 +3338,6 @@ struct fx_cdmg {
             for (fx_buf *f : {L.u, L.rhs, L.tmp, L.vx, L.vy, L.kappa}) fx_free(f);
         fx_free(tmp0);
     }
-    // Levels of at most this many points keep the separate passes in a recorded cycle: replay is for
-    // hierarchies whose cycle is many launches, and what a recording holds there is what its users
-    // count.  The fused passes would save about 5 us of a replayed cycle (127 x 127: 78 against 71 us
-    // launched directly).
-    static constexpr size_t kReplaySeparate = 2048;
     // whether level l smooths with the network in a learned cycle
     bool learned_on(size_t l) const {
         const size_t pts = lv[l].rows * lv[l].cols;
@@ -3352,8 +3347,7 @@ struct fx_cdmg {
     // scalar-kappa operator (a kappa field would need a fourth ring row array; it keeps the
     // separate passes, as other sweep counts do)
     bool fused(size_t l, bool learned) const {
-        return n_pre == 2 && n_post == 2 && !op->kappa && l + 1 < lv.size() && !(learned && learned_on(l)) &&
-               !(replay && lv[l].rows * lv[l].cols <= kReplaySeparate);
+        return n_pre == 2 && n_post == 2 && !op->kappa && l + 1 < lv.size() && !(learned && learned_on(l));
     }
     // The operator on level l: h doubled per level, the injected fields; level 0 of an F64
     // cycle reads the operator's own fields.
@@ -3519,7 +3513,11 @@ int fx_cdmg::View::apply(fx_buf *z, const fx_buf *r, const int *skip, bool z_zer
             ctx->launches++;
             return FX_OK;
         }
-    if (mg->replays.size() >= 16) return record(z, r, skip, z_zero);  // many distinct pairs: no cache
+    // This application is launched directly, and recorded behind it while the GPU works: recording and
+    // instantiating first would hold it up (FP64, 129 x 129: 104 us for the first one, from 143; 4097 x 4097
+    // 460 from 567).
+    FX_TRY(record(z, r, skip, z_zero));
+    if (mg->replays.size() >= 16) return FX_OK;  // many distinct pairs: no cache
     const size_t nf0 = ctx->deferred_free.size();
     FX_CUDA(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeRelaxed));
     const int st = record(z, r, skip, z_zero);
@@ -3533,20 +3531,18 @@ int fx_cdmg::View::apply(fx_buf *z, const fx_buf *r, const int *skip, bool z_zer
     if (st == FX_OK && e == cudaSuccess && graph && cudaGraphInstantiate(&exec, graph, 0) == cudaSuccess) {
         cudaGraphDestroy(graph);
         mg->replays.push_back({z->ptr, r->ptr, skip, z_zero, ctx->stream, exec, std::move(frees)});
-        FX_CUDA(cudaGraphLaunch(exec, ctx->stream));
-        ctx->launches++;
         return FX_OK;
     }
     if (graph) cudaGraphDestroy(graph);
     (void)cudaGetLastError();
     for (void *p : frees) cudaFreeAsync(p, ctx->stream);
-    // Not recordable here (a capture-illegal call inside, or the capture was invalidated): run
-    // the application directly, now and from now on.  A genuine error shows again in that run.
+    // Not recordable here (a capture-illegal call inside, or the capture was invalidated): every
+    // application is launched directly from now on.
     mg->replay_off = true;
-    return record(z, r, skip, z_zero);
+    return FX_OK;
 }
 
-// The launches of one application (recorded by apply, or run directly).
+// The launches of one application.
 int fx_cdmg::View::record(fx_buf *z, const fx_buf *r, const int *skip, bool z_zero) {
     CdLevel &L0 = mg->lv[0];
     const size_t n = L0.rows * L0.cols;
