@@ -700,8 +700,6 @@ int cheb_tail_top(const ChebLevel *L, int nl, size_t n_pre, size_t n_post, size_
     int top = nl;
     size_t bytes = 0;
     for (int l = nl - 1; l >= 0 && nl - l <= kChebTailLevels; l--) {
-        // the prolongation onto this level stays inside the coarser one
-        if (l + 1 < nl && ((L[l].rows - 1) / 2 > L[l + 1].rows - 1 || (L[l].cols - 1) / 2 > L[l + 1].cols - 1)) break;
         if (L[l].rows < 2 || L[l].cols < 2 || L[l].rows > kChebTailSmem || L[l].cols > kChebTailSmem) break;
         bytes += 4 * sizeof(double) * L[l].rows * L[l].cols;
         if (bytes > kChebTailSmem) break;

@@ -581,6 +581,10 @@ int reference_cycle(fx_mg *mg, fx_buf *x, const fx_buf *b, bool x_zero) {
         FX_TRY(make_stencil(&s, &P[l]));
         if (nl > 1 || mg->smoother == 1) FX_TRY(make_bc(&mg->bc, mg->lv[l].dx, mg->lv[l].dy, &B[l], true));
     }
+    // what the prolongations refuse (an odd side on a level above the coarsest), before x is touched
+    for (int l = 0; l + 1 < nl; l++)
+        if ((mg->lv[l].rows - 1) / 2 > mg->lv[l + 1].rows - 1 || (mg->lv[l].cols - 1) / 2 > mg->lv[l + 1].cols - 1)
+            return fail(FX_ERR_DIMENSION_MISMATCH, "prolong: fine grid maps outside the coarse grid");
     std::vector<ChebLevel> V;
     int top = nl;  // the levels from here on run in one block
     if (mg->smoother == 1) {
@@ -600,8 +604,6 @@ int reference_cycle(fx_mg *mg, fx_buf *x, const fx_buf *b, bool x_zero) {
         if (correct) {
             MgLevel &C = mg->lv[l + 1];
             const fx_grid g{L.rows, L.cols, L.dx, L.dy}, cg{C.rows, C.cols, C.dx, C.dy};
-            if ((g.rows - 1) / 2 > cg.rows - 1 || (g.cols - 1) / 2 > cg.cols - 1)
-                return fail(FX_ERR_DIMENSION_MISMATCH, "prolong: fine grid maps outside the coarse grid");
             if (mg->smoother == 0 || n == 0) {
                 fx_buf ub;
                 ub.ctx = ctx;
