@@ -566,8 +566,9 @@ int reference_cycle(fx_mg *mg, fx_buf *x, const fx_buf *b, bool x_zero) {
     MgLevel &L0 = mg->lv[0];
     FX_TRY(check_same(L0.rhs, b));
     FX_TRY(check_same(L0.u, x));
-    // level 0 works on the caller's x and b where they are two buffers
-    const bool own = x->ptr == b->ptr;
+    // level 0 works on the caller's x and b where they share no memory
+    const size_t bytes0 = L0.rows * L0.cols * sizeof(double);
+    const bool own = (const char *)x->ptr < (const char *)b->ptr + bytes0 && (const char *)b->ptr < (const char *)x->ptr + bytes0;
     if (own) {
         FX_TRY(fx_copy(ctx, b, L0.rhs));
         if (!x_zero) FX_TRY(fx_copy(ctx, x, L0.u));
@@ -596,7 +597,7 @@ int reference_cycle(fx_mg *mg, fx_buf *x, const fx_buf *b, bool x_zero) {
     }
     // whether level l's first smoothing takes its zero iterate as such instead of reading it
     auto zero_first = [&](int l) { return mg->smoother == 1 && (l >= top || mg->n_pre > 0 || l == nl - 1); };
-    if (x_zero && !zero_first(0)) FX_CUDA(cudaMemsetAsync(u_of(0), 0, L0.rows * L0.cols * sizeof(double), ctx->stream));
+    if (x_zero && !zero_first(0)) FX_CUDA(cudaMemsetAsync(u_of(0), 0, bytes0, ctx->stream));
     // level l's first smoothing, or the one that follows the prolongation of level l + 1's u
     auto smooth = [&](int l, size_t n, bool first) -> int {
         MgLevel &L = mg->lv[l];

@@ -27,3 +27,24 @@ def test_refused_cycle_leaves_x(dev, smoother, n):
     with pytest.raises(DimensionMismatch):
         mg.v_cycle(X, Field.from_f64(g, b, dev))
     assert np.array_equal(X.to_vec_f64(), x)
+
+
+@pytest.mark.parametrize("smoother", [0, 1])
+@pytest.mark.parametrize("shift", [5, 64, 640])
+def test_overlapping_vectors(dev, smoother, shift):
+    """x and b that share a part of their memory: the cycle is that of b as it was passed."""
+    import torch
+    from fluxion_b200 import Boundaries, DType, Field, Grid, Multigrid, SmootherKind
+    n = 128
+    g = Grid.square(n, 1.0 / (n - 1))
+    mg = Multigrid.build(g, Boundaries.zero_dirichlet(), dev, 2, 2, 2.0 / 3.0, SmootherKind(smoother))
+    om = O.Multigrid(n, n, g.dx, g.dx, 2, 2, 2.0 / 3.0, mode=0, smoother=smoother)
+    data = np.random.default_rng(shift).uniform(-1, 1, n * n + shift)
+    for xs, bs in ((0, shift), (shift, 0)):
+        t = torch.from_numpy(data).cuda()
+        torch.cuda.synchronize()
+        X, B = (Field(dev.backend().wrap(t[o:].data_ptr(), n * n, DType.F64), g, dev) for o in (xs, bs))
+        mg.v_cycle(X, B)
+        xo = data[xs:xs + n * n].copy()
+        om.v_cycle(xo, data[bs:bs + n * n].copy())
+        assert np.array_equal(X.to_vec_f64(), xo)
