@@ -3390,7 +3390,10 @@ int cd_cycle(fx_cdmg *mg, double *z, const double *r, const int *skip, bool lear
     const int nl = (int)mg->lv.size();
     constexpr bool F32 = sizeof(T) == 4;
     const size_t n0 = mg->lv[0].rows * mg->lv[0].cols;
-    const bool fused0 = mg->fused(0, learned);
+    // an F32 cycle has always taken vectors that overlap in memory: it works on copies of both
+    const bool apart = r + n0 <= z || z + n0 <= r;
+    auto fused = [&](int l) { return mg->fused(l, learned) && (l > 0 || !F32 || apart); };
+    const bool fused0 = fused(0);
     std::vector<T *> cur(nl), oth(nl);
     std::vector<const T *> rhs(nl);
     for (int l = F32 ? 0 : 1; l < nl; l++) {
@@ -3440,7 +3443,7 @@ int cd_cycle(fx_cdmg *mg, double *z, const double *r, const int *skip, bool lear
     };
     for (int l = 0; l < nl - 1; l++) {
         const CdLevel &L = mg->lv[l], &Cl = mg->lv[l + 1];
-        if (mg->fused(l, learned)) {  // x2 goes to oth[l]
+        if (fused(l)) {  // x2 goes to oth[l]
             if (F32 && l == 0)
                 FX_TRY((launch_cd_down<T, double, double>(ctx, cd_level_args<T, double, double>(mg, 0, r, oth[0], z), skip)));
             else
@@ -3455,7 +3458,7 @@ int cd_cycle(fx_cdmg *mg, double *z, const double *r, const int *skip, bool lear
         const bool coarsest = l + 1 == nl - 1;
         const size_t nc = Cl.rows * Cl.cols;
         // the next level's iterate starts from zero: a fused level and the one-block solve do so themselves
-        if (coarsest ? !(coarse_fits(nc, sizeof(T)) && mg->coarse_sweeps > 0) : !mg->fused(l + 1, learned))
+        if (coarsest ? !(coarse_fits(nc, sizeof(T)) && mg->coarse_sweeps > 0) : !fused(l + 1))
             FX_TRY(zero_fill<T>(ctx, cur[l + 1], nc, skip));
     }
     {
@@ -3476,7 +3479,7 @@ int cd_cycle(fx_cdmg *mg, double *z, const double *r, const int *skip, bool lear
     }
     for (int l = nl - 2; l >= 0; l--) {
         const CdLevel &L = mg->lv[l], &Cl = mg->lv[l + 1];
-        if (mg->fused(l, learned)) {
+        if (fused(l)) {
             if (F32 && l == 0) {
                 auto a = cd_level_args<T, double, double>(mg, 0, r, oth[0], z);
                 a.e = cur[1];
