@@ -3731,7 +3731,6 @@ int fx_mg_create(fx_ctx *ctx, const fx_grid *g, const fx_boundaries *bc, size_t 
         lap5_of(hx, hy, L.lap5);
         int st = fx_alloc(ctx, r * c, FX_F64, &L.u);
         if (!st) st = fx_alloc(ctx, r * c, FX_F64, &L.rhs);
-        if (!st) st = fx_alloc(ctx, r * c, FX_F64, &L.tmp);
         if (!st && smoother == 1) st = fx_alloc(ctx, r * c, FX_F64, &L.w0);  // multigrid.rs:113-119
         if (!st && smoother == 1) st = fx_alloc(ctx, r * c, FX_F64, &L.w1);
         mg->lv.push_back(L);

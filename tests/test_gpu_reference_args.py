@@ -48,3 +48,20 @@ def test_overlapping_vectors(dev, smoother, shift):
         xo = data[xs:xs + n * n].copy()
         om.v_cycle(xo, data[bs:bs + n * n].copy())
         assert np.array_equal(X.to_vec_f64(), xo)
+
+
+@pytest.mark.parametrize("smoother", [0, 1])
+def test_hierarchy_keeps_the_vectors_its_cycle_uses(dev, smoother):
+    """u and rhs on every level, and the Chebyshev smoother's two iterates: no vector more."""
+    import torch
+    from fluxion_b200 import Boundaries, Grid, Multigrid, SmootherKind
+    n = 4096
+    g = Grid.square(n, 1.0 / (n - 1))
+    dev.backend().synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    mg = Multigrid.build(g, Boundaries.zero_dirichlet(), dev, 2, 2, 2.0 / 3.0, SmootherKind(smoother))
+    dev.backend().synchronize()
+    taken = free - torch.cuda.mem_get_info()[0]
+    del mg
+    levels = n * n * 8 * 4 / 3
+    assert taken < ((4 if smoother else 2) + 0.5) * levels
