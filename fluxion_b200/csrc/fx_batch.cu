@@ -48,8 +48,9 @@ struct Tile {
 struct Strip {  // a warp's strip and row chunk of a fused level pass (fx_cdcycle.cuh)
     int prob, strip, nstrips, r0, r1;
 };
-// Rows per strip item: a chunk marches 5 (down) or 3 (up) rows more than it owns, so long ones are
-// cheaper a row, and short ones balance better over the resident warps.
+// Rows per strip item, at most: a chunk marches 5 (down) or 3 (up) rows more than it owns, so long ones
+// are cheaper a row, and short ones balance better over the resident warps.  A level whose items do
+// not fill the GPU takes shorter ones (strip_items).
 constexpr int kStripRows = 64;
 
 // per (level, problem): offset into the level's arrays, side n (rows = cols = n), constants
@@ -864,6 +865,33 @@ int upload_chunks(fx_batch *B, int l) {
     return FX_OK;
 }
 
+// The strip items of a level's problems (strips of `own` columns): chunks of the fewest rows with which
+// all items are resident at once (`cap` warps), of kStripRows where that is not possible; a problem's
+// chunks are of equal size.  With 64 rows throughout, a level of few or small problems was a march of
+// 64 rows by a few warps, slower than the separate tiled passes.  One FP64 cycle by separate passes,
+// with 64 rows and so, in us: 2 problems of 65 x 65 147, 170, 79; 8 of 257 x 257 251, 326, 128; 2 of
+// 1025 x 1025 412, 496, 201; 24 of 1025 x 1025 1793, 1013, 834 (more than the GPU holds: equal chunks).
+std::vector<Strip> strip_items(const std::vector<int> &probs, const std::vector<int> &side, int own, long cap) {
+    auto chunk = [](int n, int rows) {
+        const int k = (n + rows - 1) / rows;
+        return ((n + k - 1) / k + 1) & ~1;  // even
+    };
+    auto strips = [&](int n) { return (n - 1 + own - 1) / own; };
+    int rows = 2;
+    for (; rows < kStripRows; rows += 2) {
+        long items = 0;
+        for (int p : probs) items += (long)strips(side[p]) * ((side[p] + chunk(side[p], rows) - 1) / chunk(side[p], rows));
+        if (items <= cap) break;
+    }
+    std::vector<Strip> out;
+    for (int p : probs) {
+        const int n = side[p], ns = strips(n), c = chunk(n, rows);
+        for (int r0 = 0; r0 < n; r0 += c)
+            for (int s = 0; s < ns; s++) out.push_back(Strip{p, s, ns, r0, std::min(r0 + c, n)});
+    }
+    return out;
+}
+
 template <typename T>
 int build_levels(fx_batch *B) {
     const int np = (int)B->np;
@@ -883,6 +911,11 @@ int build_levels(fx_batch *B) {
     }
     B->lv.resize(B->nlev);
     const bool f32 = B->dtype == FX_F32;
+    static std::atomic<int> occ_down{0}, occ_up{0};
+    const long cap_down = (long)band_capacity(B->ctx, k_bdown<T, T>, occ_down, kCdWarps * 32,
+                                              kCdWarps * cd_down_warp_smem<T, T>()) * kCdWarps;
+    const long cap_up = (long)band_capacity(B->ctx, k_bup<T, T, T>, occ_up, kCdWarps * 32,
+                                            kCdWarps * cd_up_warp_smem<T, T>()) * kCdWarps;
     for (int l = 0; l < B->nlev; l++) {
         auto &D = B->lv[l];
         std::vector<int> have, smooth, coarse;
@@ -907,16 +940,8 @@ int build_levels(fx_batch *B) {
         FX_TRY(B->upload(&D.tiles, tiles));
         D.ntiles = (int)tiles.size();
         if (B->n_pre == 2 && B->n_post == 2) {
-            std::vector<Strip> dn, up;
-            for (int p : smooth) {
-                const int n = side[l][p];
-                const int nd = (n - 1 + kCdOwnDown - 1) / kCdOwnDown, nu = (n - 1 + kCdOwnUp - 1) / kCdOwnUp;
-                for (int r0 = 0; r0 < n; r0 += kStripRows) {
-                    const int r1 = std::min(r0 + kStripRows, n);
-                    for (int s = 0; s < nd; s++) dn.push_back(Strip{p, s, nd, r0, r1});
-                    for (int s = 0; s < nu; s++) up.push_back(Strip{p, s, nu, r0, r1});
-                }
-            }
+            const std::vector<Strip> dn = strip_items(smooth, side[l], kCdOwnDown, cap_down);
+            const std::vector<Strip> up = strip_items(smooth, side[l], kCdOwnUp, cap_up);
             FX_TRY(B->upload(&D.down, dn));
             FX_TRY(B->upload(&D.up, up));
             D.ndown = (int)dn.size();
