@@ -3213,7 +3213,9 @@ struct FlatCast {  // d = (D) s
 // loads, ten dependent operations each), so a thread has one point (PTS = 1) wherever the grid fits
 // a block: a predicated-off point still issues its instructions.  On the 17 x 17 grid 200 FP64
 // sweeps took 51 us with four point slots per thread and the coefficients read in every sweep, and
-// 42 us now.
+// 42 us now.  With four slots FP32 reads the coefficients in every sweep all the same: a V(1,1)-cycle
+// with a 34 x 34 coarsest grid takes 94 us so and 103 with them in registers, 64 x 64 173 and 192 (FP64 in
+// registers: 122 from 134, and level).
 template <typename T, int PTS>
 __global__ void __launch_bounds__(1024) k_cd_coarse(T *u, const T *__restrict__ b, int rows, int cols,
                                                     OpA<T, kModeCD> A, T omega, int nsweeps, const int *skip) {
@@ -3263,7 +3265,9 @@ __global__ void __launch_bounds__(1024) k_cd_coarse(T *u, const T *__restrict__ 
             nb.s = src[i + cols];
             nb.w = src[i - 1];
             nb.e = src[i + 1];
-            const T av = fx_fma(A.coeff, conv_diff_at<T>(A.K, nb, kv[q], xv[q], yv[q]), A.sigma * nb.c);
+            T av;
+            if constexpr (PTS > 1 && sizeof(T) == 4) av = A.apply(false, nb, (size_t)i);
+            else av = fx_fma(A.coeff, conv_diff_at<T>(A.K, nb, kv[q], xv[q], yv[q]), A.sigma * nb.c);
             dst[i] = fx_fma(omega, (bv[q] - av) * dv[q], nb.c);
         }
         __syncthreads();
