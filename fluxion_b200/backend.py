@@ -210,6 +210,20 @@ class CudaGraph:
             pass
 
 
+class DiffusionSteps:
+    """Explicit diffusion steps on u (fx_diffusion_steps) with their arguments prepared: scheme 0 Euler,
+    1 Heun, 2 RK4.  `run(n)` makes n of them."""
+
+    def __init__(self, backend: "CudaBackend", u: CudaBuffer, scratch: CudaBuffer, grid: Grid, stencil: Stencil,
+                 alpha: float, dt: float, scheme: int):
+        s, g = StencilC(stencil), grid_c(grid)
+        self._keep = (u, scratch, s, g)
+        self._args = (backend.ctx, u.handle, scratch.handle, C.byref(g), s.ptr, float(alpha), float(dt), int(scheme))
+
+    def run(self, n: int) -> None:
+        check(L.lib().fx_diffusion_steps(*self._args, int(n)))
+
+
 class CudaBackend:
     """The B200 backend: one CUDA context and stream per device."""
 
@@ -418,10 +432,7 @@ class CudaBackend:
 
     def diffusion_steps(self, u, scratch, grid: Grid, stencil: Stencil, alpha: float, dt: float, scheme: int, n: int):
         """`n` explicit diffusion steps on u (fx_diffusion_steps); scheme 0 Euler, 1 Heun, 2 RK4."""
-        s = StencilC(stencil)
-        g = grid_c(grid)
-        check(L.lib().fx_diffusion_steps(self.ctx, u.handle, scratch.handle, C.byref(g), s.ptr, float(alpha), float(dt),
-                                         int(scheme), int(n)))
+        DiffusionSteps(self, u, scratch, grid, stencil, alpha, dt, scheme).run(n)
 
     # -------------------------------------------------------------- vertex multigrid primitives
 

@@ -264,4 +264,7 @@ class Boundaries:
         return self
 
     def is_zero_dirichlet(self) -> bool:
-        return all(s.kind == BcKind.DIRICHLET and s.a == 0.0 for s in self.sides())
+        for s in (self.top, self.bottom, self.left, self.right):
+            if s.kind != BcKind.DIRICHLET or s.a != 0.0:
+                return False
+        return True

@@ -12,6 +12,7 @@ from __future__ import annotations
 import enum
 from typing import List, Optional
 
+from .backend import DiffusionSteps
 from .core import Boundaries, DType, Grid, Stencil
 from .field import Device, Field
 from .solvers import CgSolver, Multigrid, SmootherKind, SolveStats
@@ -244,8 +245,8 @@ class DiffusionSolver:
     the reference's stability bound safety * h_min^2 / (4 alpha) (safety 0.4 / 0.8 / 1.4).
     ``enable_graph()`` is the HipGraph path (solver.rs:182-325) on CUDA graphs: the first ``step_n``
     fixes the step and its field, and later calls repeat it whatever the solver's attributes are by
-    then.  A step of field operations is recorded on the backend's stream and replayed; one of the
-    fused passes is a launch or two as it is, and its arguments are kept instead."""
+    then: by replaying a recording of it or, for several steps where the fused passes hold, by the
+    passes with its arguments."""
 
     def __init__(self, grid: Grid, alpha: float, dt: Optional[float], boundaries: Boundaries,
                  scheme: "TimeScheme", device: Optional[Device] = None):
@@ -264,6 +265,7 @@ class DiffusionSolver:
         self._use_graph = False
         self._graph = None
         self._graph_u = None
+        self._graph_passes = None
 
     @staticmethod
     def new(grid: Grid, alpha: float, dt: Optional[float], device: Optional[Device] = None) -> "DiffusionSolver":
@@ -293,20 +295,21 @@ class DiffusionSolver:
         """solver.rs:182-186 (enable_hip_graph)."""
         self._use_graph = True
 
-    def _passes(self, u: Field) -> Optional[tuple]:
-        """A step of u without a source as the arguments of the library's fused passes, where these
-        hold: a five-point stencil, zero Dirichlet sides, F64 (fx_diffusion_steps; the same values as
-        the sequence of field operations)."""
+    def _passes(self, u: Field) -> Optional[DiffusionSteps]:
+        """Steps of u without a source as the library's fused passes, where these hold: a five-point
+        stencil, zero Dirichlet sides, F64 (fx_diffusion_steps; the same values as the sequence of
+        field operations)."""
         if (self.stencil.len() != 5 or not self.boundaries.is_zero_dirichlet() or u.dtype() != DType.F64
                 or u.grid() != self.grid):
             return None
         u._same(self.scratch[0])
-        return (u.storage, self.scratch[0].storage, self.grid, self.stencil, self.alpha, self._dt, self._scheme.value)
+        return DiffusionSteps(self.device.backend(), u.storage, self.scratch[0].storage, self.grid, self.stencil,
+                              self.alpha, self._dt, self._scheme.value)
 
     def step(self, u: Field, source: Optional[Field] = None) -> None:
         passes = self._passes(u) if source is None else None
         if passes is not None:
-            self.device.backend().diffusion_steps(*passes, 1)
+            passes.run(1)
         else:
             self._record(u, source)
         self._steps_done += 1
@@ -318,36 +321,40 @@ class DiffusionSolver:
             return
         n = len(range(n))  # an integer; a negative one counts as none
         if self._use_graph:
-            if self._graph is None:
-                # the fused passes have nothing to record: their arguments are the step
-                self._graph = self._passes(u)
-                if self._graph is None:
-                    be = self.device.backend()
-                    be.graph_begin()
-                    try:
-                        self._record(u, None)
-                    finally:
-                        self._graph = be.graph_end()
+            if self._graph_u is None:
+                self._graph_passes = self._passes(u)
+                if self._graph_passes is None:
+                    self._graph = self._recorded(lambda: self._record(u, None))
                 self._graph_u = u
             if u is not self._graph_u:
                 raise ValueError("the recorded step belongs to another field")
-            if isinstance(self._graph, tuple):
-                self._repeat(self._graph, n)
+            if self._graph_passes is not None and n > 1:  # fewer launches than n replays
+                self._graph_passes.run(n)
+                self._steps_done += n
                 return
+            if self._graph is None and n:
+                self._graph = self._recorded(lambda: self._graph_passes.run(1))
             for _ in range(n):
                 self._graph.launch()
                 self._steps_done += 1
             return
         passes = self._passes(u) if n else None
         if passes is not None:
-            self._repeat(passes, n)
+            passes.run(n)
+            self._steps_done += n
             return
         for _ in range(n):
-            self.step(u, None)
+            self._record(u, None)
+            self._steps_done += 1
 
-    def _repeat(self, passes: tuple, n: int) -> None:
-        self.device.backend().diffusion_steps(*passes, n)
-        self._steps_done += n
+    def _recorded(self, step):
+        be = self.device.backend()
+        be.graph_begin()
+        try:
+            step()
+        finally:
+            graph = be.graph_end()
+        return graph
 
     def step_n_with_source(self, u: Field, n: int, source: Field) -> None:
         for _ in range(n):
