@@ -22,11 +22,11 @@
 // Every point value is the expression of FlatCdSweep / FlatCdResid and the transfers, so the cycle
 // equals the unfused one bit for bit.
 //
-// Measured on a whole cycle, FP64 / FP32: 4097 x 4097 489 / 388 us (separate passes: 1062 / 857),
-// 1025 x 1025 136 / 107 (203 / 183), 65 x 65 60 / 44 (88 / 73).  The level-0 passes move 76 B/point
-// in FP64 at about 0.75 of HBM bandwidth; they are bound by the latency of a step (three dependent
-// stages of ten FP64 operations after a division) at 12 warps per SM, the levels below 513 by that
-// latency alone.
+// Measured on a whole cycle, FP64 / FP32, levels of up to 300000 points by tiles (below): 4097 x 4097
+// 448 / 354 us (separate passes: 1066 / 861), 1025 x 1025 98 / 75 (206 / 185), 65 x 65 46 / 30 (90 / 77).  The
+// level-0 passes of 4097 x 4097 move 76 B/point in FP64, down at 0.63 and up at 0.79 of the copy rate;
+// they are bound by the latency of a step (three dependent stages of ten FP64 operations after a
+// division) at 16 and 12 warps per SM.
 #pragma once
 
 #include "fx_points.cuh"
@@ -422,8 +422,8 @@ __device__ __forceinline__ void cd_up_strip(const CdLevelArgs<T, TB, TZ> &L, int
 
 // ---------------------------------------------------------------- one problem
 
-// resident blocks per SM asked of the compiler.  More of them is slower (FP64 cycle at 4097 x 4097:
-// 489 us with 3, 500 with 4 at 128 registers): the chunks get shorter, and the unrolled march is
+// resident blocks per SM asked of the compiler.  More of them is slower (FP64 cycle at 4097 x 4097 by
+// strips: 489 us with 3, 500 with 4 at 128 registers): the chunks get shorter, and the unrolled march is
 // larger than a scheduler's instruction cache, so warps at different rows evict each other's
 // instructions.  For the same reason there is no third variant of the step without column masks
 // (528 us).
@@ -472,7 +472,10 @@ constexpr int kCdTileUp = kCdTile + 4;             // halo 2: f -> x3 -> z
 constexpr int kCdTileDownThreads = (kCdTileDown * kCdTileDown + 31) / 32 * 32;
 constexpr int kCdTileUpThreads = (kCdTileUp * kCdTileUp + 31) / 32 * 32;
 // Levels up to this size go by tiles.  BiCGSTAB on 1025^2 (20 cycles) with the line at 129^2, 257^2,
-// 513^2 and 1025^2: 2967, 2836, 2759 and 3010 us; by strips alone 3490.
+// 513^2 and 1025^2: 2967, 2836, 2759 and 3010 us; by strips alone 3490.  One cycle with the finest level
+// by strips and by tiles, FP64 / FP32 in us: 321^2 62 / 47 and 52 / 38, 449^2 69 / 52 and 59 / 43, 513^2 76 / 55
+// and 66 / 47.  The crossover is between 769^2 (80 / 62 and 75 / 57) and 1025^2; the line is under it, where
+// the levels of 2^k + 1 grids leave it.
 constexpr long long kCdTilePoints = 300000;
 
 template <typename T, typename TB, typename TZ>

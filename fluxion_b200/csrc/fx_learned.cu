@@ -15,8 +15,8 @@
 // is tiled in registers: the convolutions compute 8 (or 7) points of a row x 4 channels per thread,
 // the weight gradients 8 output channels x 3 taps of a row per thread over a share of the rows.
 // Activations lie point by point with their channels adjacent, padded so that the lanes of a warp
-// (4 channel groups x 8 rows, or 16 channels) fall in distinct banks: 0.55 ms, 0.40 of the FP32 rate,
-// with 18 warps per SM and the gradient sums spilled between phases.
+// (4 channel groups x 8 rows, or 16 channels) fall in distinct banks: 0.57 ms, 0.39 of the FP32 rate
+// (0.59 ms with the call around it), with 18 warps per SM and the gradient sums spilled between phases.
 #include <algorithm>
 #include <cmath>
 #include <cstring>

@@ -655,7 +655,9 @@ int lex5_sweeps(fx_ctx *ctx, T *x, const T *b, size_t rows, size_t cols, const d
         A.nsweeps = A.nsuper > 1 ? 1 : (int)std::min<size_t>(nsweeps, (size_t)(max_warps / A.nwr));
         nsweeps -= (size_t)A.nsweeps;
         // two sweeping warps per block while the cluster has the blocks for it: the copies of four
-        // slow each other and the sweeps down (256 x 256, two sweeps: 103 us with four)
+        // slow each other and the sweeps down.  One FP64 sweep with four a block and with two: 192 x 192
+        // 55 and 52 us, 256 x 256 74 and 69, 512 x 512 157 and 138; 128 x 128, whose four warps would share
+        // one block and its barrier, 29 and 34.  FP32: 54 and 52, 73 and 70, 149 and 142, 27 and 34.
         const int warps = A.nwr * A.nsweeps;
         if (warps <= kLexMaxCta * 2) FX_TRY((lex5_launch<T, 2>(ctx, A, warps)));
         else FX_TRY((lex5_launch<T, 4>(ctx, A, warps)));

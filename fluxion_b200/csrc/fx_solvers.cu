@@ -330,7 +330,7 @@ struct fx_mg {
     fx_buf *tmp0 = nullptr;  // level-0 ping-pong partner (vertex mode)
     fx_buf *x32 = nullptr, *b32 = nullptr;  // level-0 single-precision copies (F32 cycle)
     // layout of the fused cycle (fx_mg_autotune): strip row chunks per launch in percent of one
-    // wave, and the largest level the one-block tail takes (0: as many points as it can hold)
+    // wave (levels that go by tiles have none), and the largest level the one-block tail takes (0: as many points as it can hold)
     int chunk_pct = 100;
     size_t tail_top_max = 0;
     struct View : fx_precond {
@@ -1861,7 +1861,8 @@ struct FlatGmMgs {  // w -= h_j v_j; reduction w.v_{j+1} (or w.w after the last)
 // size, and their registers are capped for two blocks per SM (three for up to 4 vectors; 5 spill at
 // three).  Against a pass per vector: 42 us an iteration of GMRES(30) at 129 x 131, from 91 (two
 // launches a step instead of k + 1), 126 from 203 at 1021 x 1531, 266 from 441 at 2049 x 2049.  The
-// dots are 14 FP64 operations for 8 bytes from HBM, 0.6 of the FP64 rate at the HBM rate.
+// dots are 14 FP64 operations for 8 bytes from HBM: 0.69 of the copy rate there (28 vectors) with the
+// FP64 pipes busy half of the time, 16 warps per SM; the update runs at the copy rate.
 constexpr int kMgsMax = 32;   // basis vectors (above, and for one vector, a pass per vector)
 constexpr int kMgsGroup = 8;  // vectors per block
 

@@ -645,7 +645,9 @@ constexpr int kTileDownThreads = (kTileDown * kTileDown + 31) / 32 * 32;
 constexpr int kTileUpThreads = (kTileUp * kTileUp + 31) / 32 * 32;
 // Levels up to this size go by tiles.  MG-PCG on 1025 x 1281 with the FP32 cycle, by strips alone and
 // with the line under 257 x 321, over it and over 1025 x 1281: 980, 957, 937 and 1154 us; on 4097^2 in
-// FP64 with the line under 513^2 and over it: 4150 and 4163 us.
+// FP64 with the line under 513^2 and over it: 4150 and 4163 us, which is level.  One cycle with the
+// finest level by strips and by tiles, FP64 / FP32 in us: 257^2 53 / 41 and 48 / 37, 385^2 52 / 43 and 47 / 39,
+// 513^2 61 / 48 and 56 / 44 (over the line: a solve's finest up pass, with r.z, marches strips anyway).
 constexpr size_t kTilePoints = 150000;
 
 template <typename T, typename TB>
