@@ -1856,15 +1856,16 @@ struct FlatGmMgs {  // w -= h_j v_j; reduction w.v_{j+1} (or w.w after the last)
 // 60 iterations: 6.67e-16 relative in the mean here, 6.64e-16 with a pass per vector; attained
 // residuals on operators of condition 1e7 to 1e8 (200 of them): 0.99 of the others' in the mean.
 //
-// Dots: a block takes a group of up to 8 basis vectors (its threads hold 8 pairs of sums) over a
+// Dots: a block takes a group of up to 6 basis vectors (its threads hold 6 pairs of sums) over a
 // share of the elements, so w and v_k are read once per group, mostly from L2; groups are of equal
 // size, and their registers are capped for two blocks per SM (three for up to 4 vectors; 5 spill at
-// three).  Against a pass per vector: 42 us an iteration of GMRES(30) at 129 x 131, from 91 (two
-// launches a step instead of k + 1), 126 from 203 at 1021 x 1531, 266 from 441 at 2049 x 2049.  The
-// dots are 14 FP64 operations for 8 bytes from HBM: 0.69 of the copy rate there (28 vectors) with the
-// FP64 pipes busy half of the time, 16 warps per SM; the update runs at the copy rate.
+// three).  Groups of up to 8 spill a little (266 us an iteration of GMRES(30) at 2049 x 2049, 257 with 6,
+// 265 with 5, 277 with 4).  Against a pass per vector: 43 us an iteration at 129 x 131, from 91 (two
+// launches a step instead of k + 1), 122 from 203 at 1021 x 1531, 257 from 441 at 2049 x 2049.  The
+// dots are 14 FP64 operations for 8 bytes from HBM: 0.76 of the copy rate there (26 to 30 vectors) with
+// the FP64 pipes busy 58 % of the time, 16 warps per SM; the update runs at the copy rate.
 constexpr int kMgsMax = 32;   // basis vectors (above, and for one vector, a pass per vector)
-constexpr int kMgsGroup = 8;  // vectors per block
+constexpr int kMgsGroup = 6;  // vectors per block
 
 struct MgsArgs {
     double *w;
@@ -2076,9 +2077,7 @@ int mgs_two_pass(fx_gmres *s, size_t n, double *w, const std::vector<double *> &
         case 3: FX_TRY(launch_mgs_dots<3>(ctx, n, a)); break;
         case 4: FX_TRY(launch_mgs_dots<4>(ctx, n, a)); break;
         case 5: FX_TRY(launch_mgs_dots<5>(ctx, n, a)); break;
-        case 6: FX_TRY(launch_mgs_dots<6>(ctx, n, a)); break;
-        case 7: FX_TRY(launch_mgs_dots<7>(ctx, n, a)); break;
-        default: FX_TRY(launch_mgs_dots<8>(ctx, n, a)); break;
+        default: FX_TRY(launch_mgs_dots<6>(ctx, n, a)); break;
     }
     static std::atomic<int> occ{0};
     const size_t cap = (size_t)band_capacity(ctx, k_mgs_update, occ, kBlock);
